@@ -33,6 +33,7 @@
 // as thick in physical units.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
@@ -44,7 +45,9 @@
 
 #include "../../include/pflbm.h"
 #include "engine.h"
+#include "gridbar.cuh"
 #include "kernels.cuh"
+#include "packed.cuh"
 
 namespace {
 
@@ -82,7 +85,9 @@ __host__ __device__ inline uint64_t mix64(uint64_t x) {
     return x;
 }
 
-__device__ __forceinline__ float sigmoidf_(float a) { return 1.0f / (1.0f + expf(-a)); }
+// (the correctly rounded reciprocal is the correctly rounded quotient 1 / x,
+// in fewer instructions than a division)
+__device__ __forceinline__ float sigmoidf_(float a) { return __frcp_rn(1.0f + expf(-a)); }
 
 // ------------------------------------------------------------- data
 __global__ void k_filter_restrict(const float *__restrict__ macro, uint64_t Nf, int nxf, int nyf, int nzf, int nxc,
@@ -324,26 +329,41 @@ __global__ void __launch_bounds__(kSB) k_mlp_grad(const float *__restrict__ blob
 }
 
 // ------------------------------------------- network on the tensor cores
-// The same forward + backward over kSB = 128 samples per CTA with every
+// The same forward + backward over blocks of kSB = 128 samples with every
 // matrix product on the tensor cores: warp-level mma.m16n8k8 with TF32
 // operands (10-bit mantissa, operands rounded to nearest) and FP32
-// accumulation. Warp w owns samples 32w .. 32w+31 (two 16-row tiles):
-//   layer 1   A1 = Xn W1^T + b1       (16 x 8 x 8 per tile and column block)
+// accumulation. A pair of warps owns 32 samples, each warp one 16-row tile
+// of them up to the weight gradients, whose output rows they then share:
+//   layer 1   A1 = Xn W1^T + b1       (16 x 8 x 8 per column block)
 //   layer 2   A2 = H1 W2^T + b2       (K = 32: four k steps)
 //   backward  dH1 = dA2 W2            (K = 32)
-//   weights   dW2 = dA2^T H1, dW1 = dA1^T Xn   (K = the warp's 32 samples)
+//   weights   dW2 = dA2^T H1, dW1 = dA1^T Xn   (K = the pair's 32 samples)
 // and the elementwise parts (SiLU, softplus, bias and w3 sums) in FP32. The
-// four warps' partial gradients are summed in warp order: gpart is filled
-// as k_mlp_grad fills it (sums over the CTA's samples, loss last).
-constexpr int kTcWarps = kSB / 32;
-constexpr int kTcX = 12;                 // row stride of the Xn tile (floats)
-constexpr int kTcH = kMlpH + 4;          // row stride of the 32-wide tiles
-constexpr int kTcWarpFloats = 32 * kTcX + 3 * 32 * kTcH + 32;  // Xn, H1, dA2, dA1, dz
-constexpr int kTcPart = kMlpParams + 1;  // per-warp partial gradient + loss
-
-size_t tc_smem_bytes() {
-    return sizeof(float) * (size_t(kMlpBlob) + size_t(kTcWarps) * kTcWarpFloats + size_t(kTcWarps) * kTcPart);
-}
+// four pairs' partial gradients are summed in pair order in FP32 (the block's
+// gradient, as k_mlp_grad's) and added to the CTA's FP64 sums.
+//
+// What bounds it is the dependent chain of one block (gather, two layers,
+// two layers back, column sums), not the 112 MMAs per 32 samples. So the
+// weights are laid out once as TF32 fragments in lane order (8-byte
+// conflict-free loads instead of 4- and 8-way conflicts and a conversion per
+// use), a sigmoid is evaluated once per unit instead of two or three times,
+// and two warps share what one warp did: 2^20 samples 398 -> 226 us (IPC 1.6
+// at 16 warps per SM; 3640 warp instructions per 32 samples).
+constexpr int kTcThreads = 2 * kSB;
+constexpr int kTcPairs = kSB / 32;
+constexpr int kTcX = 12;         // row stride of the Xn tile (words)
+constexpr int kTcH = kMlpH + 4;  // row stride of the 32-wide tiles
+// shared words: weight fragments and constants, then per pair Xn, H1 (TF32
+// bits), dA2, dA1, dz, loss, the w3 sums of the first tile, then the pairs'
+// partial gradients
+constexpr int kTcF1 = 0, kTcF2 = kTcF1 + 256, kTcF2T = kTcF2 + 1024, kTcB1 = kTcF2T + 1024, kTcB2 = kTcB1 + kMlpH,
+              kTcW3 = kTcB2 + kMlpH, kTcMean = kTcW3 + kMlpH, kTcInv = kTcMean + kMlpIn, kTcB3 = kTcInv + kMlpIn,
+              kTcScale = kTcB3 + 1, kTcWeights = kTcB3 + 4;
+constexpr int kTcPairWords = 32 * kTcX + 3 * 32 * kTcH + 32 + 32 + 8 * 32;
+constexpr int kTcPart = kMlpParams + 1;  // partial gradient + loss
+constexpr int kTcAcc = (kTcPart + kTcThreads - 1) / kTcThreads;  // FP64 sums per thread
+constexpr int kTcSmem = 4 * (kTcWeights + kTcPairs * kTcPairWords + kTcPairs * kTcPart);
+static_assert(kMlpH == 32 && kMlpIn == 8, "fragment layout");
 
 __device__ __forceinline__ uint32_t to_tf32(float x) {
     uint32_t r;
@@ -352,213 +372,259 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 }
 
 // D = A B + C, A 16x8 (row), B 8x8 (col), TF32 operands, FP32 accumulators.
-__device__ __forceinline__ void mma_tf32_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                              uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_tf32_1688(float (&d)[4], const uint32_t (&a)[4], uint2 b) {
     asm volatile(
         "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
         "{%0, %1, %2, %3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
 }
 
-__device__ __forceinline__ float silu_grad(float a) {
-    const float sg = sigmoidf_(a);
-    return sg * (1.0f + a * (1.0f - sg));
+// The two warps of a pair (named barriers 1 .. kTcPairs; 0 is the block's).
+__device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); }
+
+// The blob as fragments: B operand words of lane (g = lane / 4, t = lane % 4)
+// side by side, W1 and W2 by output column block and k step, W2 once more
+// transposed for the backward product. Read past the L1, which another CTA's
+// update of the blob does not invalidate.
+__device__ __forceinline__ void tc_load_weights(float *s, const float *blob) {
+    uint32_t *w = reinterpret_cast<uint32_t *>(s);
+    constexpr int kPer = (kMlpBlob + kTcThreads - 1) / kTcThreads;
+    float got[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+        if (threadIdx.x + kTcThreads * k < kMlpBlob) got[k] = __ldcg(blob + threadIdx.x + kTcThreads * k);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int i = threadIdx.x + kTcThreads * k;
+        const float v = got[k];
+        if (i < pflbm::kMlpB1) {
+            const int n = i >> 3, k = i & 7;
+            w[kTcF1 + (((n >> 3) * 32 + (n & 7) * 4 + (k & 3)) * 2) + (k >> 2)] = to_tf32(v);
+        } else if (i < pflbm::kMlpW2) {
+            s[kTcB1 + i - pflbm::kMlpB1] = v;
+        } else if (i < pflbm::kMlpB2) {
+            const int j = (i - pflbm::kMlpW2) >> 5, c = (i - pflbm::kMlpW2) & 31;
+            const uint32_t b = to_tf32(v);
+            w[kTcF2 + (((j >> 3) * 4 + (c >> 3)) * 32 + (j & 7) * 4 + (c & 3)) * 2 + ((c >> 2) & 1)] = b;
+            w[kTcF2T + (((c >> 3) * 4 + (j >> 3)) * 32 + (c & 7) * 4 + (j & 3)) * 2 + ((j >> 2) & 1)] = b;
+        } else if (i < pflbm::kMlpW3) {
+            s[kTcB2 + i - pflbm::kMlpB2] = v;
+        } else if (i < pflbm::kMlpB3) {
+            s[kTcW3 + i - pflbm::kMlpW3] = v;
+        } else if (i == pflbm::kMlpB3) {
+            s[kTcB3] = v;
+        } else if (i < pflbm::kMlpInvScale) {
+            s[kTcMean + i - pflbm::kMlpMean] = v;
+        } else if (i < pflbm::kMlpOutScale) {
+            s[kTcInv + i - pflbm::kMlpInvScale] = v;
+        } else if (i == pflbm::kMlpOutScale) {
+            s[kTcScale] = v;
+        }
+    }
 }
 
-__global__ void __launch_bounds__(kSB) k_mlp_grad_tc(const float *__restrict__ blob, const float *__restrict__ X,
-                                                     const float *__restrict__ Y, uint64_t n, int mode,
-                                                     uint64_t seed, uint64_t iter, uint64_t count,
-                                                     float *__restrict__ gpart) {
-    extern __shared__ float tcs[];
-    float *w = tcs;
+// What a warp needs of its 16 samples of a block: lane l half a row (row
+// l / 2) of features, lanes 0 .. 15 the target of row l.
+struct TcRows {
+    float4 x;
+    float y;
+    bool vx, vy;  // the rows exist (the last block is ragged)
+};
+
+__device__ __forceinline__ TcRows tc_fetch(const float *__restrict__ X, const float *__restrict__ Y, uint64_t n,
+                                           int mode, uint64_t seed, uint64_t iter, uint64_t count, int block) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    float *base = tcs + kMlpBlob + warp * kTcWarpFloats;
-    float *xs = base;                       // [32][kTcX]
-    float *h1s = xs + 32 * kTcX;            // [32][kTcH]
-    float *da2s = h1s + 32 * kTcH;          // [32][kTcH]
-    float *da1s = da2s + 32 * kTcH;         // [32][kTcH]
-    float *dzs = da1s + 32 * kTcH;          // [32]
-    float *part = tcs + kMlpBlob + kTcWarps * kTcWarpFloats + warp * kTcPart;
-    for (int i = threadIdx.x; i < kMlpBlob; i += kSB) w[i] = blob[i];
-    __syncthreads();
-    const float out_scale = w[pflbm::kMlpOutScale];
-
-    // this lane's sample (row `lane` of the warp's tile): normalised features
-    const uint64_t k = blockIdx.x * uint64_t(kSB) + threadIdx.x;
-    const bool valid = k < count;
+    const uint64_t base = uint64_t(block) * kSB + uint64_t(warp) * 16;
+    TcRows r{make_float4(0.f, 0.f, 0.f, 0.f), 0.0f, base + (lane >> 1) < count, lane < 16 && base + lane < count};
+    const uint64_t k = base + (lane >> 1);
     uint64_t idx = 0;
-    if (valid) idx = mode == 0 ? k : mix64(seed * 0x9E3779B97F4A7C15ull + mix64(iter * 0x100000001B3ull + k)) % n;
-    for (int q = 0; q < kMlpIn; ++q)
-        xs[lane * kTcX + q] = valid ? (X[idx * kMlpIn + q] - w[pflbm::kMlpMean + q]) * w[pflbm::kMlpInvScale + q]
-                                    : 0.0f;
-    const float target = valid ? Y[idx] / out_scale : 0.0f;
+    if (r.vx) idx = mode == 0 ? k : mix64(seed * 0x9E3779B97F4A7C15ull + mix64(iter * 0x100000001B3ull + k)) % n;
+    if (r.vx) r.x = __ldg(reinterpret_cast<const float4 *>(X + idx * kMlpIn) + (lane & 1));
+    const uint64_t iy = __shfl_sync(0xffffffffu, idx, (2 * lane) & 31);
+    if (r.vy) r.y = __ldg(Y + iy);
+    return r;
+}
+
+// Gradient of one block's samples, added to the calling thread's FP64 sums
+// (parameter threadIdx.x + kTcThreads j in acc[j]; the loss is the last one).
+__device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&acc)[kTcAcc]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pair = warp >> 1, half = warp & 1;  // this warp's rows: 16 half .. 16 half + 15 of the pair's 32
+    const int g = lane >> 2, t = lane & 3;
+    float *base = s + kTcWeights + pair * kTcPairWords;
+    uint32_t *xs = reinterpret_cast<uint32_t *>(base);  // [32][kTcX], TF32
+    uint32_t *h1s = xs + 32 * kTcX;                     // [32][kTcH], TF32
+    float *da2s = base + 32 * kTcX + 32 * kTcH;         // [32][kTcH]
+    float *da1s = da2s + 32 * kTcH;                     // [32][kTcH]
+    float *dzs = da1s + 32 * kTcH;                      // [32]
+    float *losses = dzs + 32;                           // [32]
+    float *w3p = losses + 32;                           // [8][32]
+    float *part = s + kTcWeights + kTcPairs * kTcPairWords + pair * kTcPart;
+    const uint2 *f1 = reinterpret_cast<const uint2 *>(s + kTcF1), *f2 = reinterpret_cast<const uint2 *>(s + kTcF2),
+                *f2t = reinterpret_cast<const uint2 *>(s + kTcF2T);
+
+    // normalised features
+    {
+        const int q = 4 * (lane & 1);
+        const float *mean = s + kTcMean + q, *inv = s + kTcInv + q;
+        const float4 x = rows.x;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (rows.vx)
+            v = make_uint4(to_tf32((x.x - mean[0]) * inv[0]), to_tf32((x.y - mean[1]) * inv[1]),
+                           to_tf32((x.z - mean[2]) * inv[2]), to_tf32((x.w - mean[3]) * inv[3]));
+        *reinterpret_cast<uint4 *>(&xs[(16 * half + (lane >> 1)) * kTcX + q]) = v;
+    }
+    const float target = rows.vy ? rows.y / s[kTcScale] : 0.0f;
     __syncwarp();
 
-    // layer 1: a1 = Xn W1^T + b1 (fragments: rows 16 mt + g (+8), columns
-    // 8 nt + 2 t (+1)); h1 = SiLU(a1) to shared memory
-    float a1[2][4][4], a2[2][4][4];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    const int r0 = 16 * half + g;  // fragment rows r0 and r0 + 8, columns 8 nt + 2 t (+1)
+    // layer 1: a1 = Xn W1^T + b1; h1 = SiLU(a1) to shared memory, SiLU'(a1) kept
+    float sg1[4][4];
+    {
+        const uint32_t a[4] = {xs[r0 * kTcX + t], xs[(r0 + 8) * kTcX + t], xs[r0 * kTcX + t + 4],
+                               xs[(r0 + 8) * kTcX + t + 4]};
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            float(&d)[4] = a1[mt][nt];
-            d[0] = d[2] = w[pflbm::kMlpB1 + 8 * nt + 2 * t];
-            d[1] = d[3] = w[pflbm::kMlpB1 + 8 * nt + 2 * t + 1];
-            const int r0 = 16 * mt + g;
-            mma_tf32_1688(d, to_tf32(xs[r0 * kTcX + t]), to_tf32(xs[(r0 + 8) * kTcX + t]),
-                          to_tf32(xs[r0 * kTcX + t + 4]), to_tf32(xs[(r0 + 8) * kTcX + t + 4]),
-                          to_tf32(w[pflbm::kMlpW1 + (8 * nt + g) * kMlpIn + t]),
-                          to_tf32(w[pflbm::kMlpW1 + (8 * nt + g) * kMlpIn + t + 4]));
+            const float c0 = s[kTcB1 + 8 * nt + 2 * t], c1 = s[kTcB1 + 8 * nt + 2 * t + 1];
+            float d[4] = {c0, c1, c0, c1};
+            mma_tf32_1688(d, a, f1[nt * 32 + lane]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int row = r0 + (e >= 2 ? 8 : 0), col = 8 * nt + 2 * t + (e & 1);
-                h1s[row * kTcH + col] = d[e] * sigmoidf_(d[e]);
+                const float sg = sigmoidf_(d[e]);
+                h1s[(r0 + (e >= 2 ? 8 : 0)) * kTcH + 8 * nt + 2 * t + (e & 1)] = to_tf32(d[e] * sg);
+                sg1[nt][e] = sg * (1.0f + d[e] * (1.0f - sg));
             }
         }
+    }
     __syncwarp();
     // layer 2: a2 = H1 W2^T + b2; z = w3 . SiLU(a2) + b3 per sample
-    float zp[2][2] = {{0.f, 0.f}, {0.f, 0.f}};  // [mt][row g / g + 8], this lane's columns
+    float h2[4][4], sg2[4][4], zp[2] = {0.f, 0.f};
+    {
+        uint32_t a[4][4];
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+        for (int kk = 0; kk < 4; ++kk) {
+            a[kk][0] = h1s[r0 * kTcH + 8 * kk + t];
+            a[kk][1] = h1s[(r0 + 8) * kTcH + 8 * kk + t];
+            a[kk][2] = h1s[r0 * kTcH + 8 * kk + t + 4];
+            a[kk][3] = h1s[(r0 + 8) * kTcH + 8 * kk + t + 4];
+        }
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            float(&d)[4] = a2[mt][nt];
-            d[0] = d[2] = w[pflbm::kMlpB2 + 8 * nt + 2 * t];
-            d[1] = d[3] = w[pflbm::kMlpB2 + 8 * nt + 2 * t + 1];
-            const int r0 = 16 * mt + g;
+            const float c0 = s[kTcB2 + 8 * nt + 2 * t], c1 = s[kTcB2 + 8 * nt + 2 * t + 1];
+            float d[4] = {c0, c1, c0, c1};
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-                mma_tf32_1688(d, to_tf32(h1s[r0 * kTcH + 8 * kk + t]), to_tf32(h1s[(r0 + 8) * kTcH + 8 * kk + t]),
-                              to_tf32(h1s[r0 * kTcH + 8 * kk + t + 4]),
-                              to_tf32(h1s[(r0 + 8) * kTcH + 8 * kk + t + 4]),
-                              to_tf32(w[pflbm::kMlpW2 + (8 * nt + g) * kMlpH + 8 * kk + t]),
-                              to_tf32(w[pflbm::kMlpW2 + (8 * nt + g) * kMlpH + 8 * kk + t + 4]));
+            for (int kk = 0; kk < 4; ++kk) mma_tf32_1688(d, a[kk], f2[(nt * 4 + kk) * 32 + lane]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int col = 8 * nt + 2 * t + (e & 1);
-                zp[mt][e >> 1] += w[pflbm::kMlpW3 + col] * (d[e] * sigmoidf_(d[e]));
+                const float sg = sigmoidf_(d[e]);
+                h2[nt][e] = d[e] * sg;
+                sg2[nt][e] = sg * (1.0f + d[e] * (1.0f - sg));
+                zp[e >> 1] = __fmaf_rn(s[kTcW3 + 8 * nt + 2 * t + (e & 1)], h2[nt][e], zp[e >> 1]);
             }
         }
+    }
     // complete z over the 4 lanes of a group, then dz per row to shared memory
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            zp[mt][h] += __shfl_xor_sync(0xffffffffu, zp[mt][h], 1);
-            zp[mt][h] += __shfl_xor_sync(0xffffffffu, zp[mt][h], 2);
-        }
+    for (int h = 0; h < 2; ++h) {
+        zp[h] += __shfl_xor_sync(0xffffffffu, zp[h], 1);
+        zp[h] += __shfl_xor_sync(0xffffffffu, zp[h], 2);
+    }
     if (t == 0) {
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) dzs[16 * mt + g + 8 * h] = zp[mt][h] + w[pflbm::kMlpB3];
+        dzs[r0] = zp[0] + s[kTcB3];
+        dzs[r0 + 8] = zp[1] + s[kTcB3];
     }
     __syncwarp();
-    // this lane's own sample: loss and dz
-    float loss_l, dz_l;
-    {
-        const float z = dzs[lane];
+    if (lane < 16) {
+        const float z = dzs[16 * half + lane];
         const float sp = fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z)));
-        const float r = valid ? sp - target : 0.0f;
-        loss_l = valid ? r * r : 0.0f;
-        dz_l = valid ? 2.0f * r * sigmoidf_(z) : 0.0f;
+        const float r = rows.vy ? sp - target : 0.0f;
+        losses[16 * half + lane] = rows.vy ? r * r : 0.0f;
+        dzs[16 * half + lane] = rows.vy ? 2.0f * r * sigmoidf_(z) : 0.0f;
     }
     __syncwarp();
-    dzs[lane] = dz_l;
-    __syncwarp();
-    // backward: dA2 = dz w3 SiLU'(a2); dw3 partials over this lane's rows
-    float dw3p[4][2] = {};
+    // backward: dA2 = dz w3 SiLU'(a2); the w3 sums of the pair run over the
+    // first warp's rows, then over the second's
+    const float dz0 = dzs[r0], dz1 = dzs[r0 + 8];
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int e = 0; e < 4; ++e) {
+            const int col = 8 * nt + 2 * t + (e & 1);
+            da2s[(r0 + (e >= 2 ? 8 : 0)) * kTcH + col] = (e >= 2 ? dz1 : dz0) * s[kTcW3 + col] * sg2[nt][e];
+        }
+    if (half == 0) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int row = 16 * mt + g + (e >= 2 ? 8 : 0), col = 8 * nt + 2 * t + (e & 1);
-                const float dz = dzs[row], av = a2[mt][nt][e];
-                da2s[row * kTcH + col] = dz * w[pflbm::kMlpW3 + col] * silu_grad(av);
-                dw3p[nt][e & 1] += dz * (av * sigmoidf_(av));
-            }
+        for (int k = 0; k < 8; ++k)
+            w3p[k * 32 + lane] = __fmaf_rn(dz1, h2[k >> 1][2 + (k & 1)], __fmul_rn(dz0, h2[k >> 1][k & 1]));
+    }
     __syncwarp();
     // dH1 = dA2 W2, dA1 = dH1 SiLU'(a1)
+    {
+        uint32_t a[4][4];
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+        for (int kk = 0; kk < 4; ++kk) {
+            a[kk][0] = to_tf32(da2s[r0 * kTcH + 8 * kk + t]);
+            a[kk][1] = to_tf32(da2s[(r0 + 8) * kTcH + 8 * kk + t]);
+            a[kk][2] = to_tf32(da2s[r0 * kTcH + 8 * kk + t + 4]);
+            a[kk][3] = to_tf32(da2s[(r0 + 8) * kTcH + 8 * kk + t + 4]);
+        }
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
             float d[4] = {0.f, 0.f, 0.f, 0.f};
-            const int r0 = 16 * mt + g;
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-                mma_tf32_1688(d, to_tf32(da2s[r0 * kTcH + 8 * kk + t]), to_tf32(da2s[(r0 + 8) * kTcH + 8 * kk + t]),
-                              to_tf32(da2s[r0 * kTcH + 8 * kk + t + 4]),
-                              to_tf32(da2s[(r0 + 8) * kTcH + 8 * kk + t + 4]),
-                              to_tf32(w[pflbm::kMlpW2 + (8 * kk + t) * kMlpH + 8 * nt + g]),
-                              to_tf32(w[pflbm::kMlpW2 + (8 * kk + t + 4) * kMlpH + 8 * nt + g]));
+            for (int kk = 0; kk < 4; ++kk) mma_tf32_1688(d, a[kk], f2t[(nt * 4 + kk) * 32 + lane]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int row = r0 + (e >= 2 ? 8 : 0), col = 8 * nt + 2 * t + (e & 1);
-                da1s[row * kTcH + col] = d[e] * silu_grad(a1[mt][nt][e]);
-            }
+            for (int e = 0; e < 4; ++e)
+                da1s[(r0 + (e >= 2 ? 8 : 0)) * kTcH + 8 * nt + 2 * t + (e & 1)] = d[e] * sg1[nt][e];
         }
-    __syncwarp();
-    // weight gradients over the warp's 32 samples (K)
+    }
+    pair_sync(pair);
+    // weight gradients over the pair's 32 samples (K): this warp the output
+    // rows 16 half .. 16 half + 15
+    {
+        uint32_t a[4][4];
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
+        for (int kk = 0; kk < 4; ++kk) {
+            a[kk][0] = to_tf32(da2s[(8 * kk + t) * kTcH + r0]);
+            a[kk][1] = to_tf32(da2s[(8 * kk + t) * kTcH + r0 + 8]);
+            a[kk][2] = to_tf32(da2s[(8 * kk + t + 4) * kTcH + r0]);
+            a[kk][3] = to_tf32(da2s[(8 * kk + t + 4) * kTcH + r0 + 8]);
+        }
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {  // dW2[j][i] = sum_s dA2[s][j] H1[s][i]
             float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                mma_tf32_1688(d, to_tf32(da2s[(8 * kk + t) * kTcH + 16 * mt + g]),
-                              to_tf32(da2s[(8 * kk + t) * kTcH + 16 * mt + g + 8]),
-                              to_tf32(da2s[(8 * kk + t + 4) * kTcH + 16 * mt + g]),
-                              to_tf32(da2s[(8 * kk + t + 4) * kTcH + 16 * mt + g + 8]),
-                              to_tf32(h1s[(8 * kk + t) * kTcH + 8 * nt + g]),
-                              to_tf32(h1s[(8 * kk + t + 4) * kTcH + 8 * nt + g]));
+                mma_tf32_1688(d, a[kk], make_uint2(h1s[(8 * kk + t) * kTcH + 8 * nt + g],
+                                                   h1s[(8 * kk + t + 4) * kTcH + 8 * nt + g]));
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int j = 16 * mt + g + (e >= 2 ? 8 : 0), i = 8 * nt + 2 * t + (e & 1);
-                part[pflbm::kMlpW2 + j * kMlpH + i] = d[e];
-            }
+            for (int e = 0; e < 4; ++e)
+                part[pflbm::kMlpW2 + (r0 + (e >= 2 ? 8 : 0)) * kMlpH + 8 * nt + 2 * t + (e & 1)] = d[e];
         }
         float d[4] = {0.f, 0.f, 0.f, 0.f};  // dW1[i][q] = sum_s dA1[s][i] Xn[s][q]
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-            mma_tf32_1688(d, to_tf32(da1s[(8 * kk + t) * kTcH + 16 * mt + g]),
-                          to_tf32(da1s[(8 * kk + t) * kTcH + 16 * mt + g + 8]),
-                          to_tf32(da1s[(8 * kk + t + 4) * kTcH + 16 * mt + g]),
-                          to_tf32(da1s[(8 * kk + t + 4) * kTcH + 16 * mt + g + 8]),
-                          to_tf32(xs[(8 * kk + t) * kTcX + g]), to_tf32(xs[(8 * kk + t + 4) * kTcX + g]));
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int i = 16 * mt + g + (e >= 2 ? 8 : 0), q = 2 * t + (e & 1);
-            part[pflbm::kMlpW1 + i * kMlpIn + q] = d[e];
+        for (int kk = 0; kk < 4; ++kk) {
+            const uint32_t b[4] = {to_tf32(da1s[(8 * kk + t) * kTcH + r0]), to_tf32(da1s[(8 * kk + t) * kTcH + r0 + 8]),
+                                   to_tf32(da1s[(8 * kk + t + 4) * kTcH + r0]),
+                                   to_tf32(da1s[(8 * kk + t + 4) * kTcH + r0 + 8])};
+            mma_tf32_1688(d, b, make_uint2(xs[(8 * kk + t) * kTcX + g], xs[(8 * kk + t + 4) * kTcX + g]));
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            part[pflbm::kMlpW1 + (r0 + (e >= 2 ? 8 : 0)) * kMlpIn + 2 * t + (e & 1)] = d[e];
     }
-    // bias and w3 gradients, loss: column sums over the warp's samples
+    // bias gradients: column sums over the pair's samples, b1 by the first
+    // warp, b2 by the second
     {
-        float sb1 = 0.f, sb2 = 0.f;
-        for (int s = 0; s < 32; ++s) {
-            sb1 += da1s[s * kTcH + lane];
-            sb2 += da2s[s * kTcH + lane];
-        }
-        part[pflbm::kMlpB1 + lane] = sb1;
-        part[pflbm::kMlpB2 + lane] = sb2;
+        const float *col = (half == 0 ? da1s : da2s) + lane;
+        float sum = 0.f;
+#pragma unroll
+        for (int r = 0; r < 32; ++r) sum += col[r * kTcH];
+        part[(half == 0 ? pflbm::kMlpB1 : pflbm::kMlpB2) + lane] = sum;
     }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            float v = dw3p[nt][c];
-            v += __shfl_xor_sync(0xffffffffu, v, 4);
-            v += __shfl_xor_sync(0xffffffffu, v, 8);
-            v += __shfl_xor_sync(0xffffffffu, v, 16);
-            if (g == 0) part[pflbm::kMlpW3 + 8 * nt + 2 * t + c] = v;
-        }
-    {
-        float sdz = dz_l, sl = loss_l;
+    if (half == 0) {
+        float sdz = dzs[lane], sl = losses[lane];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             sdz += __shfl_xor_sync(0xffffffffu, sdz, o);
@@ -568,19 +634,173 @@ __global__ void __launch_bounds__(kSB) k_mlp_grad_tc(const float *__restrict__ b
             part[pflbm::kMlpB3] = sdz;
             part[kMlpParams] = sl;
         }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float v = __fmaf_rn(dz0, h2[k >> 1][k & 1], w3p[k * 32 + lane]);
+            v = __fmaf_rn(dz1, h2[k >> 1][2 + (k & 1)], v);
+            v += __shfl_xor_sync(0xffffffffu, v, 4);
+            v += __shfl_xor_sync(0xffffffffu, v, 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 16);
+            if (g == 0) part[pflbm::kMlpW3 + 8 * (k >> 1) + 2 * t + (k & 1)] = v;
+        }
     }
     __syncthreads();
-    // the block's sums, warps in order
-    float *gout = gpart + size_t(blockIdx.x) * (kMlpParams + 1);
-    const float *parts = tcs + kMlpBlob + kTcWarps * kTcWarpFloats;
-    for (int p = threadIdx.x; p <= kMlpParams; p += kSB) {
-        float acc = 0.0f;
+    // the block's sums, pairs in order
+    const float *parts = s + kTcWeights + kTcPairs * kTcPairWords;
 #pragma unroll
-        for (int ww = 0; ww < kTcWarps; ++ww) acc += parts[ww * kTcPart + p];
-        gout[p] = acc;
+    for (int j = 0; j < kTcAcc; ++j) {
+        const int p = threadIdx.x + kTcThreads * j;
+        if (p <= kMlpParams) {
+            float v = 0.0f;
+#pragma unroll
+            for (int q = 0; q < kTcPairs; ++q) v += parts[q * kTcPart + p];
+            acc[j] += v;
+        }
+    }
+    __syncthreads();
+}
+
+// One parameter's sum over the CTAs' rows of gsum[cta][kTcPart], for the
+// kSumP parameters from p0 on: 16 groups of threads take every 16th row each,
+// then the groups are added in order. Every parameter's rows are in flight at
+// once; one thread per parameter and row after row took 20 us for 128 rows
+// and 1.16 ms for 8192. The sum is the return value of the threads of group 0
+// (tid < kSumP; parameter p0 + tid).
+constexpr int kSumP = 16, kSumG = kTcThreads / kSumP;
+constexpr int kSumCtas = (kTcPart + kSumP - 1) / kSumP;  // CTAs that cover all parameters
+
+__device__ __forceinline__ double tc_sum_rows(const double *gsum, int rows, int p0, double *red) {
+    const int p = p0 + int(threadIdx.x) % kSumP, grp = int(threadIdx.x) / kSumP;
+    double v = 0.0;
+    if (p <= kMlpParams) {
+#pragma unroll 8
+        for (int r = grp; r < rows; r += kSumG) v += __ldcg(gsum + size_t(r) * kTcPart + p);
+    }
+    red[threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.x < kSumP) {
+        double q[4];  // four short chains: an FP64 addition takes about 60 cycles here
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = red[k * kSumP + threadIdx.x];
+#pragma unroll
+        for (int k = 4; k < kSumG; ++k) q[k & 3] += red[k * kSumP + threadIdx.x];
+        v = (q[0] + q[1]) + (q[2] + q[3]);
+    }
+    return v;
+}
+
+// Gradient of the first `count` samples: every CTA runs its share of the
+// blocks and writes its FP64 sums as a row of gsum; k_grad_rows adds the rows.
+__global__ void __launch_bounds__(kTcThreads, 2) k_mlp_grad_tc(const float *__restrict__ blob,
+                                                               const float *__restrict__ X,
+                                                               const float *__restrict__ Y, uint64_t n,
+                                                               uint64_t count, int blocks, double *__restrict__ gsum) {
+    extern __shared__ __align__(16) float tcs[];
+    tc_load_weights(tcs, blob);
+    double acc[kTcAcc] = {};
+    TcRows rows = tc_fetch(X, Y, n, 0, 0, 0, count, blockIdx.x);
+    __syncthreads();
+    for (int b = blockIdx.x; b < blocks; b += gridDim.x) {
+        const TcRows now = rows;
+        // the next block's samples arrive while this one is computed
+        if (b + int(gridDim.x) < blocks) rows = tc_fetch(X, Y, n, 0, 0, 0, count, b + gridDim.x);
+        tc_block(tcs, now, acc);
+    }
+#pragma unroll
+    for (int j = 0; j < kTcAcc; ++j) {
+        const int p = threadIdx.x + kTcThreads * j;
+        if (p <= kMlpParams) gsum[size_t(blockIdx.x) * kTcPart + p] = acc[j];
     }
 }
 
+__global__ void __launch_bounds__(kTcThreads) k_grad_rows(const double *gsum, int rows, double *__restrict__ grad) {
+    __shared__ double red[kTcThreads];
+    const double v = tc_sum_rows(gsum, rows, blockIdx.x * kSumP, red);
+    const int p = blockIdx.x * kSumP + threadIdx.x;
+    if (threadIdx.x < kSumP && p <= kMlpParams) grad[p] = v;
+}
+
+// Adam on one parameter, rounded op by op (no contraction left to the
+// compiler), so that every kernel that calls it moves a parameter alike.
+__device__ __forceinline__ void adam_update(float g, float lr, float beta1, float beta2, float eps, float c1, float c2,
+                                            float &m, float &v, float &w) {
+    m = __fmaf_rn(1.0f - beta1, g, __fmul_rn(beta1, m));
+    v = __fmaf_rn(__fmul_rn(1.0f - beta2, g), g, __fmul_rn(beta2, v));
+    w = __fsub_rn(w, __fdiv_rn(__fmul_rn(lr, __fdiv_rn(m, c1)), __fadd_rn(__fsqrt_rn(__fdiv_rn(v, c2)), eps)));
+}
+
+// A stretch of training iterations in ONE cooperative launch. An iteration is
+// short (a few us) and strictly serial, so launches and a sum over the blocks
+// by a few threads were most of it. Here every CTA keeps its place: gradient
+// of its blocks into its row of gsum, grid barrier, Adam on the 16 parameters
+// that the CTA owns (moments in registers), grid barrier, the new blob as
+// fragments. The next iteration's samples do not depend on the parameters and
+// are fetched while the CTA waits at the first barrier. 16 384 samples per iteration: 36 us
+// (two launches) -> 13 us: the block 6.1, its FP64 row and the sums 2.5, the
+// barriers 3, the weights 0.8.
+constexpr int kTrainChunk = 128;  // iterations per launch
+struct TrainArgs {
+    float *blob, *m, *v;
+    const float *X, *Y;
+    uint64_t n, seed, iter0, count;
+    int blocks, iterations, log0;
+    float inv_count, lr, beta1, beta2, eps;
+    double *gsum, *loss_log;
+    unsigned int *arrived;  // the launch's grid barriers, 0 before it
+    unsigned int *err;
+    float c1[kTrainChunk], c2[kTrainChunk];  // 1 - beta^t of the bias corrections
+};
+
+__global__ void __launch_bounds__(kTcThreads, 2) k_mlp_train(const __grid_constant__ TrainArgs a) {
+    extern __shared__ __align__(16) float tcs[];
+    __shared__ double red[kTcThreads];
+    __shared__ int s_ok;
+    const int p = blockIdx.x * kSumP + threadIdx.x;
+    const bool owner = threadIdx.x < kSumP && p < kMlpParams;
+    float m = 0.0f, v = 0.0f, w = 0.0f;
+    if (owner) m = a.m[p], v = a.v[p], w = a.blob[p];
+    const int rows_used = min(int(gridDim.x), a.blocks);  // the CTAs that have a block
+    const bool has = int(blockIdx.x) < a.blocks;
+    TcRows rows{};
+    if (has) rows = tc_fetch(a.X, a.Y, a.n, 1, a.seed, a.iter0, a.count, blockIdx.x);
+    for (int it = 0; it < a.iterations; ++it) {
+        tc_load_weights(tcs, a.blob);
+        __syncthreads();
+        if (has) {
+            double acc[kTcAcc] = {};
+            for (int b = blockIdx.x; b < a.blocks; b += gridDim.x) {
+                const TcRows now = rows;
+                if (b + int(gridDim.x) < a.blocks)
+                    rows = tc_fetch(a.X, a.Y, a.n, 1, a.seed, a.iter0 + it, a.count, b + gridDim.x);
+                tc_block(tcs, now, acc);
+            }
+#pragma unroll
+            for (int j = 0; j < kTcAcc; ++j) {
+                const int k = threadIdx.x + kTcThreads * j;
+                if (k <= kMlpParams) __stcg(a.gsum + size_t(blockIdx.x) * kTcPart + k, acc[j]);
+            }
+        }
+        pflbm::grid_arrive(a.arrived);
+        if (has && it + 1 < a.iterations) rows = tc_fetch(a.X, a.Y, a.n, 1, a.seed, a.iter0 + it + 1, a.count, blockIdx.x);
+        if (!pflbm::grid_wait(a.arrived, gridDim.x, 2 * it, a.err, &s_ok)) return;
+        if (blockIdx.x < kSumCtas) {
+            const double s = tc_sum_rows(a.gsum, rows_used, blockIdx.x * kSumP, red);
+            if (owner) {
+                const float g = float(s) * a.inv_count;
+                adam_update(g, a.lr, a.beta1, a.beta2, a.eps, a.c1[it], a.c2[it], m, v, w);
+                __stcg(a.blob + p, w);
+            } else if (threadIdx.x < kSumP && p == kMlpParams) {
+                a.loss_log[a.log0 + it] = s * a.inv_count;
+            }
+        }
+        pflbm::grid_arrive(a.arrived);
+        if (!pflbm::grid_wait(a.arrived, gridDim.x, 2 * it + 1, a.err, &s_ok)) return;
+    }
+    if (owner) a.m[p] = m, a.v[p] = v;
+}
+
+// ---- the FP32 CUDA-core kernel's sums (PFLBM_MLP_SIMT=1)
 // Sums the block gradients (fixed order, FP64) into grad[0..kMlpParams]
 // (the last entry is the loss sum).
 __global__ void k_grad_sum(const float *__restrict__ gpart, int nblocks, double *__restrict__ grad) {
@@ -604,31 +824,77 @@ __global__ void k_adam(float *__restrict__ blob, float *__restrict__ m, float *_
         return;
     }
     const float g = float(s) * inv_count;
-    const float mm = beta1 * m[p] + (1.0f - beta1) * g;
-    const float vv = beta2 * v[p] + (1.0f - beta2) * g * g;
-    m[p] = mm;
-    v[p] = vv;
-    blob[p] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+    adam_update(g, lr, beta1, beta2, eps, c1, c2, m[p], v[p], blob[p]);
 }
 
-// Forward only: FP64 loss sum per block.
-__global__ void __launch_bounds__(256) k_mlp_loss(const float *__restrict__ blob, const float *__restrict__ X,
-                                                  const float *__restrict__ Y, uint64_t n, double *__restrict__ partial) {
-    __shared__ float w[kMlpBlob];
-    for (int i = threadIdx.x; i < kMlpBlob; i += blockDim.x) w[i] = blob[i];
+// Forward only: FP64 loss sum per block. A thread evaluates two samples at a
+// time with packed FP32x2 arithmetic, the weights in shared memory twice side
+// by side so that one 16-byte broadcast feeds two packed multiply-adds: the
+// one-sample form issued a shared load per multiply-add and spilled its
+// activations (255 registers). Each sample rounds as mlp_nu_t does. 2^20
+// samples: 376 -> 130 us.
+constexpr int kLossThreads = 128;
+__global__ void __launch_bounds__(kLossThreads, 4) k_mlp_loss(const float *__restrict__ blob, const float *__restrict__ X,
+                                                           const float *__restrict__ Y, uint64_t n,
+                                                           double *__restrict__ partial) {
+    using pflbm::V2;
+    __shared__ __align__(16) float2 w[kMlpBlob];
+    for (int i = threadIdx.x; i < kMlpBlob; i += kLossThreads) w[i] = make_float2(blob[i], blob[i]);
     __syncthreads();
+    auto w2 = [&](int i, V2 &a, V2 &b) {  // weights i and i + 1, i even
+        const float4 v = *reinterpret_cast<const float4 *>(&w[i]);
+        a = V2(v.x, v.y);
+        b = V2(v.z, v.w);
+    };
+    auto silu2 = [](V2 a) { return V2(pflbm::silu_d<float>(a.v.x), pflbm::silu_d<float>(a.v.y)); };
+    static_assert(pflbm::kMlpW1 % 2 == 0 && pflbm::kMlpW2 % 2 == 0, "pairs of weights");
+    const float out_scale = w[pflbm::kMlpOutScale].x;
     double acc = 0.0;
-    for (uint64_t s = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; s < n; s += uint64_t(gridDim.x) * blockDim.x) {
-        float x[kMlpIn];
-        for (int q = 0; q < kMlpIn; ++q) x[q] = X[s * kMlpIn + q];
-        const float nu = pflbm::mlp_nu_t<float>(w, x);
-        const float r = (nu - Y[s]) / w[pflbm::kMlpOutScale];
-        acc += double(r) * r;
+    const uint64_t pairs = (n + 1) / 2;
+    for (uint64_t k = blockIdx.x * uint64_t(kLossThreads) + threadIdx.x; k < pairs;
+         k += uint64_t(gridDim.x) * kLossThreads) {
+        asm volatile("" ::: "memory");  // keeps the weight loads inside the loop (hoisted, they spill)
+        const bool second = 2 * k + 1 < n;
+        const float4 *xa = reinterpret_cast<const float4 *>(X + 2 * k * kMlpIn), *xb = second ? xa + 2 : xa;
+        const float4 a0 = xa[0], a1 = xa[1], b0 = xb[0], b1 = xb[1];
+        V2 xn[kMlpIn] = {V2(a0.x, b0.x), V2(a0.y, b0.y), V2(a0.z, b0.z), V2(a0.w, b0.w),
+                         V2(a1.x, b1.x), V2(a1.y, b1.y), V2(a1.z, b1.z), V2(a1.w, b1.w)};
+#pragma unroll
+        for (int q = 0; q < kMlpIn; ++q)
+            xn[q] = (xn[q] - V2(w[pflbm::kMlpMean + q])) * V2(w[pflbm::kMlpInvScale + q]);
+        V2 h1[kMlpH];
+#pragma unroll
+        for (int i = 0; i < kMlpH; ++i) {
+            V2 s(w[pflbm::kMlpB1 + i]), wa, wb;
+#pragma unroll
+            for (int q = 0; q < kMlpIn; q += 2) {
+                w2(pflbm::kMlpW1 + i * kMlpIn + q, wa, wb);
+                s = pflbm::fma2(wb, xn[q + 1], pflbm::fma2(wa, xn[q], s));
+            }
+            h1[i] = silu2(s);
+        }
+        V2 z(w[pflbm::kMlpB3]);
+#pragma unroll 2
+        for (int j = 0; j < kMlpH; ++j) {
+            V2 s(w[pflbm::kMlpB2 + j]), wa, wb;
+#pragma unroll
+            for (int i = 0; i < kMlpH; i += 2) {
+                w2(pflbm::kMlpW2 + j * kMlpH + i, wa, wb);
+                s = pflbm::fma2(wb, h1[i + 1], pflbm::fma2(wa, h1[i], s));
+            }
+            z = pflbm::fma2(V2(w[pflbm::kMlpW3 + j]), silu2(s), z);
+        }
+        const float ra = (out_scale * pflbm::softplus_d<float>(z.v.x) - Y[2 * k]) / out_scale;
+        acc += double(ra) * ra;
+        if (second) {
+            const float rb = (out_scale * pflbm::softplus_d<float>(z.v.y) - Y[2 * k + 1]) / out_scale;
+            acc += double(rb) * rb;
+        }
     }
-    __shared__ double sh[256];
+    __shared__ double sh[kLossThreads];
     sh[threadIdx.x] = acc;
     __syncthreads();
-    for (int st = 128; st > 0; st >>= 1) {
+    for (int st = kLossThreads / 2; st > 0; st >>= 1) {
         if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
         __syncthreads();
     }
@@ -644,8 +910,11 @@ struct pflbm_closure {
     uint64_t cap = 0, n = 0;
     float *X = nullptr, *Y = nullptr;
     float *blob = nullptr, *m = nullptr, *v = nullptr;
-    float *gpart = nullptr;
+    float *gpart = nullptr;  // per-block gradients of the CUDA-core kernel
     int gpart_blocks = 0;
+    double *gsum = nullptr;  // per-CTA gradient sums of the tensor-core kernels
+    int grad_ctas = 0;       // resident CTAs of the tensor-core kernels: rows of gsum
+    unsigned int *sync = nullptr;  // grid barrier count and error word of the training kernel
     double *grad = nullptr, *partial = nullptr, *loss_log = nullptr;
     int loss_log_cap = 0;
     float *coarse = nullptr;
@@ -658,7 +927,7 @@ struct pflbm_closure {
 
     ~pflbm_closure() {
         cudaSetDevice(device);
-        void *ptrs[] = {X, Y, blob, m, v, gpart, grad, partial, loss_log, coarse, width_part};
+        void *ptrs[] = {X, Y, blob, m, v, gpart, gsum, sync, grad, partial, loss_log, coarse, width_part};
         for (void *p : ptrs)
             if (p) cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
@@ -694,21 +963,34 @@ int download_blob(pflbm_closure *c) {
 
 size_t act_bytes() { return sizeof(Act); }
 
-// Gradient kernel of a training step: the tensor-core kernel, or with
-// PFLBM_MLP_SIMT=1 the FP32 CUDA-core kernel (exact FP32 products, for
-// checks against the FP64 oracle at FP32 rounding).
+// Gradients by the tensor-core kernels, or with PFLBM_MLP_SIMT=1 by the FP32
+// CUDA-core kernel (exact FP32 products, for checks against the FP64 oracle at
+// FP32 rounding).
 bool use_simt_grad() {
     const char *e = std::getenv("PFLBM_MLP_SIMT");
     return e && e[0] == '1';
 }
 
-void launch_grad(pflbm_closure *c, int blocks, int mode, uint64_t seed, uint64_t iter, uint64_t count) {
-    if (use_simt_grad())
-        k_mlp_grad<<<blocks, kSB, act_bytes(), c->stream>>>(c->blob, c->X, c->Y, c->n, mode, seed, iter, count,
-                                                            c->gpart);
-    else
-        k_mlp_grad_tc<<<blocks, kSB, tc_smem_bytes(), c->stream>>>(c->blob, c->X, c->Y, c->n, mode, seed, iter,
-                                                                   count, c->gpart);
+void launch_grad_simt(pflbm_closure *c, int blocks, int mode, uint64_t seed, uint64_t iter, uint64_t count) {
+    k_mlp_grad<<<blocks, kSB, act_bytes(), c->stream>>>(c->blob, c->X, c->Y, c->n, mode, seed, iter, count, c->gpart);
+}
+
+// Iterations it0 .. it0 + k - 1 of a training call in one cooperative launch:
+// one CTA per block as far as they are all resident, and never fewer than
+// own all parameters.
+cudaError_t launch_train(pflbm_closure *c, TrainArgs &a) {
+    const int grid = std::max(kSumCtas, std::min(a.blocks, c->grad_ctas));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = kTcSmem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_mlp_train, a);
 }
 
 }  // namespace
@@ -738,15 +1020,27 @@ int pflbm_closure_create(int32_t device, uint64_t max_samples, pflbm_closure **o
         cudaMalloc(&c->v, sizeof(float) * kMlpParams) != cudaSuccess ||
         cudaMalloc(&c->grad, sizeof(double) * (kMlpParams + 1)) != cudaSuccess ||
         cudaMalloc(&c->partial, sizeof(double) * kLossBlocks * 18) != cudaSuccess ||
+        cudaMalloc(&c->sync, 2 * sizeof(unsigned int)) != cudaSuccess ||
         cudaMalloc(&c->width_part, sizeof(double) * kMakeBlocks * 4) != cudaSuccess) {
         cudaGetLastError();
         return fail(PFLBM_ERR_OUT_OF_MEMORY, "closure buffers");
     }
     if (cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, int(act_bytes())) != cudaSuccess)
         return cuda_fail(cudaGetLastError(), "k_mlp_grad shared memory");
-    if (cudaFuncSetAttribute(k_mlp_grad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tc_smem_bytes())) !=
-        cudaSuccess)
-        return cuda_fail(cudaGetLastError(), "k_mlp_grad_tc shared memory");
+    if (cudaFuncSetAttribute(k_mlp_grad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
+        return cuda_fail(cudaGetLastError(), "gradient kernel shared memory");
+    // both kernels run at most as many CTAs as are resident at once
+    int sms = 0, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mlp_train, kTcThreads, kTcSmem) != cudaSuccess ||
+        sms * per_sm < kSumCtas)
+        return cuda_fail(cudaGetLastError(), "training kernel occupancy");
+    c->grad_ctas = sms * per_sm;
+    if (cudaMalloc(&c->gsum, sizeof(double) * size_t(c->grad_ctas) * kTcPart) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(PFLBM_ERR_OUT_OF_MEMORY, "closure buffers");
+    }
     *out = c.release();
     return PFLBM_OK;
 }
@@ -916,9 +1210,15 @@ int pflbm_closure_gradient(pflbm_closure *c, uint64_t count, double *host_grad, 
     if (!c->have_params) return fail(PFLBM_ERR_STATE, "closure parameters not initialised");
     cudaSetDevice(c->device);
     const int blocks = int((count + kSB - 1) / kSB);
-    if (int rc = ensure_gpart(c, blocks)) return rc;
-    launch_grad(c, blocks, 0, 0, 0, count);
-    k_grad_sum<<<(kMlpParams + 1 + 255) / 256, 256, 0, c->stream>>>(c->gpart, blocks, c->grad);
+    if (use_simt_grad()) {
+        if (int rc = ensure_gpart(c, blocks)) return rc;
+        launch_grad_simt(c, blocks, 0, 0, 0, count);
+        k_grad_sum<<<(kMlpParams + 1 + 255) / 256, 256, 0, c->stream>>>(c->gpart, blocks, c->grad);
+    } else {
+        const int ctas = std::min(blocks, c->grad_ctas);
+        k_mlp_grad_tc<<<ctas, kTcThreads, kTcSmem, c->stream>>>(c->blob, c->X, c->Y, c->n, count, blocks, c->gsum);
+        k_grad_rows<<<kSumCtas, kTcThreads, 0, c->stream>>>(c->gsum, ctas, c->grad);
+    }
     std::vector<double> g(kMlpParams + 1);
     cudaError_t e = cudaMemcpyAsync(g.data(), c->grad, sizeof(double) * g.size(), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -934,8 +1234,10 @@ int pflbm_closure_train(pflbm_closure *c, int32_t iterations, int32_t batch, flo
     if (!c->have_params) return fail(PFLBM_ERR_STATE, "closure parameters not initialised");
     if (c->n == 0) return fail(PFLBM_ERR_STATE, "no training samples");
     cudaSetDevice(c->device);
-    const int blocks = (batch + kSB - 1) / kSB;
-    if (int rc = ensure_gpart(c, blocks)) return rc;
+    const int blocks = int((int64_t(batch) + kSB - 1) / kSB);
+    const bool simt = use_simt_grad();
+    if (simt)
+        if (int rc = ensure_gpart(c, blocks)) return rc;
     if (c->loss_log_cap < iterations) {
         if (c->loss_log) cudaFree(c->loss_log);
         c->loss_log = nullptr;
@@ -947,17 +1249,44 @@ int pflbm_closure_train(pflbm_closure *c, int32_t iterations, int32_t batch, flo
         c->loss_log_cap = iterations;
     }
     const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
-    for (int it = 0; it < iterations; ++it) {
-        const uint64_t t = ++c->adam_t;
-        const float c1 = float(1.0 - std::pow(double(beta1), double(t)));
-        const float c2 = float(1.0 - std::pow(double(beta2), double(t)));
-        launch_grad(c, blocks, 1, seed, t, uint64_t(batch));
-        k_adam<<<(kMlpParams + 1 + 255) / 256, 256, 0, c->stream>>>(c->blob, c->m, c->v, c->gpart, blocks,
-                                                                   1.0f / float(batch), lr, beta1, beta2, eps, c1, c2,
-                                                                   c->loss_log, it);
+    auto correction = [](float beta, uint64_t t) { return float(1.0 - std::pow(double(beta), double(t))); };
+    if (simt) {
+        for (int it = 0; it < iterations; ++it) {
+            const uint64_t t = ++c->adam_t;
+            launch_grad_simt(c, blocks, 1, seed, t, uint64_t(batch));
+            k_adam<<<(kMlpParams + 1 + 255) / 256, 256, 0, c->stream>>>(
+                c->blob, c->m, c->v, c->gpart, blocks, 1.0f / float(batch), lr, beta1, beta2, eps,
+                correction(beta1, t), correction(beta2, t), c->loss_log, it);
+        }
+    } else {
+        TrainArgs a{};
+        a.blob = c->blob, a.m = c->m, a.v = c->v, a.X = c->X, a.Y = c->Y;
+        a.n = c->n, a.seed = seed, a.count = uint64_t(batch), a.blocks = blocks;
+        a.inv_count = 1.0f / float(batch), a.lr = lr, a.beta1 = beta1, a.beta2 = beta2, a.eps = eps;
+        a.gsum = c->gsum, a.loss_log = c->loss_log, a.arrived = c->sync, a.err = c->sync + 1;
+        cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned int), c->stream);
+        for (int it = 0; it < iterations; it += kTrainChunk) {
+            a.iterations = std::min(kTrainChunk, iterations - it);
+            a.iter0 = c->adam_t + 1;
+            a.log0 = it;
+            for (int k = 0; k < a.iterations; ++k) {
+                a.c1[k] = correction(beta1, a.iter0 + k);
+                a.c2[k] = correction(beta2, a.iter0 + k);
+            }
+            c->adam_t += a.iterations;
+            if (it > 0) cudaMemsetAsync(c->sync, 0, sizeof(unsigned int), c->stream);
+            const cudaError_t le = launch_train(c, a);
+            if (le != cudaSuccess) return cuda_fail(le, "training launch");
+        }
     }
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "closure training");
+    if (!simt) {
+        unsigned int w = 0;
+        e = cudaMemcpy(&w, c->sync + 1, sizeof w, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return cuda_fail(e, "closure training");
+        if (w) return fail(PFLBM_ERR_DEVICE, "the training kernel gave up waiting at its grid barrier");
+    }
     if (loss_history) {
         e = cudaMemcpy(loss_history, c->loss_log, sizeof(double) * iterations, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "loss history");
@@ -969,7 +1298,7 @@ int pflbm_closure_loss(pflbm_closure *c, double *mean_loss) {
     if (!c || !mean_loss) return fail(PFLBM_ERR_INVALID_ARG, "null argument");
     if (!c->have_params || c->n == 0) return fail(PFLBM_ERR_STATE, "no parameters or samples");
     cudaSetDevice(c->device);
-    k_mlp_loss<<<kLossBlocks, 256, 0, c->stream>>>(c->blob, c->X, c->Y, c->n, c->partial);
+    k_mlp_loss<<<kLossBlocks, kLossThreads, 0, c->stream>>>(c->blob, c->X, c->Y, c->n, c->partial);
     std::vector<double> part(kLossBlocks);
     cudaError_t e = cudaMemcpyAsync(part.data(), c->partial, sizeof(double) * kLossBlocks, cudaMemcpyDeviceToHost,
                                     c->stream);

@@ -21,6 +21,7 @@
 
 #include "../../include/pflbm.h"
 #include "engine_impl.cuh"
+#include "gridbar.cuh"
 
 namespace pflbm {
 
@@ -32,15 +33,6 @@ struct BoxDev {
 
 struct WorkItem {
     int box, x0, y0, zb, ze;
-};
-
-// Grid-wide barrier of the fused step (self-resetting: the last CTA to
-// arrive clears the count and advances the generation).
-struct GridBar {
-    unsigned int count;
-    unsigned int gen;
-    unsigned int never;  // the test build's flag that nothing sets
-    unsigned int pad;
 };
 
 struct BatchPtrs {
@@ -132,64 +124,6 @@ struct BatchStages {
 };
 template <int QQ, class G>
 using BatchLayout = TmaPlan<QQ, float, BatchStages<QQ, G>::value, float, G>;
-
-// Bounded polls of the grid barrier (with a short sleep each: well above any
-// sweep's duration, below a second).
-constexpr uint32_t kGridWaitLimit = 1u << 22;
-
-__device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int *p) {
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Grid-wide barrier of a cooperative launch, every poll bounded: on a
-// timeout the CTA sets bit 2 of the error word and gets false (the caller
-// returns; CTAs still waiting on it time out the same way). Thread 0 makes
-// the CTA's writes visible (fence after the block barrier) before arriving.
-// The test build -DPFLBM_TEST_DEAD_GRID waits instead on a flag that
-// nothing sets, with a short limit.
-__device__ __forceinline__ bool grid_barrier(GridBar *gb, unsigned int nblocks, unsigned int *err, int *s_ok) {
-    __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        bool ok = true;
-        const unsigned int g0 = ld_acquire_gpu(&gb->gen);
-        __threadfence();
-        const unsigned int arrived = atomicAdd(&gb->count, 1u) + 1u;
-#ifdef PFLBM_TEST_DEAD_GRID
-        (void)arrived;
-        (void)nblocks;
-        (void)g0;
-        ok = false;
-        for (uint32_t i = 0; i < (1u << 12); ++i)
-            if (ld_acquire_gpu(&gb->never) != 0u) {
-                ok = true;
-                break;
-            }
-        if (!ok) atomicOr(err, 2u);
-#else
-        if (arrived == nblocks) {
-            atomicExch(&gb->count, 0u);
-            __threadfence();
-            atomicAdd(&gb->gen, 1u);
-        } else {
-            ok = false;
-            for (uint32_t i = 0; i < kGridWaitLimit; ++i) {
-                if (ld_acquire_gpu(&gb->gen) != g0) {
-                    ok = true;
-                    break;
-                }
-                __nanosleep(64);
-            }
-            if (!ok) atomicOr(err, 2u);
-        }
-#endif
-        __threadfence();
-        *s_ok = ok ? 1 : 0;
-    }
-    __syncthreads();
-    return *s_ok != 0;
-}
 
 // One whole time step of every box in ONE launch (cooperative: all CTAs are
 // resident): the TMA-fed collide sweep over the work items (the tile code of
