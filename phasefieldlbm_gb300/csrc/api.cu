@@ -195,23 +195,6 @@ namespace {
 using pflbm::derive;
 using pflbm::validate;
 
-int pick_zchunk(const pflbm_config &c, int device) {
-    if (const char *e = std::getenv("PFLBM_ZCHUNK")) {
-        const int v = std::atoi(e);
-        if (v > 0) return v;
-    }
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int ctas_xy = int((c.nx + pflbm::kTileX - 1) / pflbm::kTileX) * int((c.ny + pflbm::kTileY - 1) / pflbm::kTileY);
-    const int nzi = int(c.nz) - 2;
-    int chunks = (8 * sms + ctas_xy - 1) / ctas_xy;
-    if (chunks < 1) chunks = 1;
-    int zc = (nzi + chunks - 1) / chunks;
-    if (zc < 4) zc = 4;
-    if (zc > nzi) zc = nzi;
-    return zc;
-}
-
 void destroy_graphs(pflbm_sim *s) {
     for (auto &row : s->graphs)
         for (auto &g : row)
@@ -524,7 +507,7 @@ int pflbm_create(const pflbm_config *cfg, pflbm_sim **out) {
     if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
     s->device = dev;
     derive(*cfg, s->hp);
-    s->hp.zchunk = pick_zchunk(*cfg, dev);
+    cudaDeviceGetAttribute(&s->hp.sms, cudaDevAttrMultiProcessorCount, dev);
     const bool jet = cfg->flow_case == PFLBM_CASE_JET;
     Engine *eng = nullptr;
     switch (cfg->storage) {

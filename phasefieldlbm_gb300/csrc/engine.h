@@ -14,7 +14,7 @@ namespace pflbm {
 struct HostParams {
     uint32_t nx, ny, nz;
     uint64_t N;
-    int32_t zchunk;
+    int32_t sms;  // multiprocessors of the device
     double sigma, gamma, u_inf, omega_ref;
     double tau_water, tau_oil, visc_water, visc_oil, kgain1, omco_zmin;
     double z_start, inv_nz_m1, inv_sponge;

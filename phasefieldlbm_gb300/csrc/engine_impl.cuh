@@ -22,7 +22,7 @@ Params<T> make_params(const HostParams &h) {
     p.nx = h.nx; p.ny = h.ny; p.nz = h.nz;
     p.plane = h.nx * h.ny;
     p.N = h.N;
-    p.zchunk = h.zchunk;
+    p.zchunk = 1;  // set for a kernel by pick_zchunk
     // FP32 runs use the float-rounded constants exactly as the reference
     // computes them; FP64 runs use the double values.
     p.sigma = f ? T(h.f_sigma) : T(h.sigma);
@@ -170,7 +170,52 @@ class EngineT final : public Engine {
             return PFLBM_ERR_CUDA;
         }
         setup_tma();
+        choose_zchunk();
         return PFLBM_OK;
+    }
+
+    // z chunks of the step's collide kernel and of the analysis kernel
+    // (pick_zchunk); PFLBM_ZCHUNK overrides both.
+    template <class K>
+    int zchunk_for(K *kernel, int threads, size_t smem) const {
+        const int nzi = int(h_.nz) - 2;
+        if (const char *e = std::getenv("PFLBM_ZCHUNK")) {
+            const int v = std::atoi(e);
+            if (v > 0) return v;
+        }
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1) {
+            cudaGetLastError();
+            per_sm = 1;
+        }
+        return pick_zchunk(int(((h_.nx + TX - 1) / TX) * ((h_.ny + TY - 1) / TY)), nzi, h_.sms, per_sm);
+    }
+    void choose_zchunk() {
+        const size_t sm = TmaLayout<QQ, S>::total;
+        if constexpr (sizeof(S) >= 4) {
+            const size_t smc = TmaModeLayout<QQ, S, MODE_STEP_CLOSURE>::total + closure_smem_bytes<T>();
+            if (closure_ && use_tma_ && tma_closure_)
+                p_.zchunk = avg_ ? zchunk_for(k_collide_tma<QQ, JET, S, MODE_STEP_CLOSURE_AVG>, NT, smc)
+                                 : zchunk_for(k_collide_tma<QQ, JET, S, MODE_STEP_CLOSURE>, NT, smc);
+            else if (closure_)
+                p_.zchunk = avg_ ? zchunk_for(k_collide<QQ, JET, S, MODE_STEP_CLOSURE_AVG>, NT, 0)
+                                 : zchunk_for(k_collide<QQ, JET, S, MODE_STEP_CLOSURE>, NT, 0);
+        }
+        if (!closure_) {
+            if (use_tma_ && avg_) {
+                p_.zchunk = zchunk_for(k_collide_tma<QQ, JET, S, MODE_STEP_AVG>, NT, sm);
+            } else if (use_pair_) {
+                if constexpr (sizeof(T) == 4)
+                    p_.zchunk = zchunk_for(k_collide_pair<QQ, JET, S>, NT2, PairLayout<QQ, S>::total);
+            } else if (use_tma_) {
+                p_.zchunk = zchunk_for(k_collide_tma<QQ, JET, S, MODE_STEP>, NT, sm);
+            } else {
+                p_.zchunk = avg_ ? zchunk_for(k_collide<QQ, JET, S, MODE_STEP_AVG>, NT, 0)
+                                 : zchunk_for(k_collide<QQ, JET, S, MODE_STEP>, NT, 0);
+            }
+        }
+        pa_ = p_;
+        pa_.zchunk = zchunk_for(k_collide<QQ, JET, S, MODE_ANALYSIS>, NT, 0);
     }
 
     // The TMA collide kernel needs 16-byte aligned row strides; otherwise the
@@ -257,9 +302,10 @@ class EngineT final : public Engine {
         return b;
     }
 
-    dim3 collide_grid() const {
+    dim3 collide_grid() const { return collide_grid(p_); }
+    dim3 collide_grid(const Params<T> &p) const {
         const int nzi = int(h_.nz) - 2;
-        const int chunks = (nzi + p_.zchunk - 1) / p_.zchunk;
+        const int chunks = (nzi + p.zchunk - 1) / p.zchunk;
         return dim3((h_.nx + TX - 1) / TX, (h_.ny + TY - 1) / TY, chunks);
     }
     dim3 node_block() const { return dim3(32, 8, 1); }
@@ -342,7 +388,7 @@ class EngineT final : public Engine {
         b.step_in = nullptr;
         b.step_out = nullptr;
         b.t_fixed = t;
-        k_collide<QQ, JET, S, MODE_ANALYSIS><<<collide_grid(), dim3(TX, TY, 1), 0, s>>>(p_, b);
+        k_collide<QQ, JET, S, MODE_ANALYSIS><<<collide_grid(pa_), dim3(TX, TY, 1), 0, s>>>(pa_, b);
         k_analysis_ghosts<T><<<node_grid(), node_block(), 0, s>>>(p_, JET ? 1 : 0, t, macro_);
     }
     void enqueue_vorticity(cudaStream_t s) override {
@@ -381,6 +427,7 @@ class EngineT final : public Engine {
         } else {
             if (!host_blob) {
                 closure_ = false;
+                choose_zchunk();
                 return PFLBM_OK;
             }
             if (!mlp_) {
@@ -397,6 +444,7 @@ class EngineT final : public Engine {
                 return PFLBM_ERR_CUDA;
             }
             closure_ = true;
+            choose_zchunk();
             return PFLBM_OK;
         }
     }
@@ -417,7 +465,7 @@ class EngineT final : public Engine {
     static constexpr int kRedBlocks = 608;
     HostParams h_;
     uint32_t flags_;
-    Params<T> p_;
+    Params<T> p_, pa_;  // of the step's kernels; of the analysis kernel (its own z chunk)
     S *f_[2] = {nullptr, nullptr};
     T *phi_[2] = {nullptr, nullptr};
     T *j_ = nullptr, *top_ = nullptr, *macro_ = nullptr, *avg_ = nullptr, *vort_ = nullptr;

@@ -572,8 +572,11 @@ int pflbm_ensemble_create(const pflbm_config *cfgs, int32_t n, pflbm_ensemble **
     uint64_t f_off = 0, n_off = 0;
     for (int k = 0; k < n; ++k) {
         pflbm::derive(cfgs[k], e->hps[k]);
-        e->hps[k].zchunk = e->zchunk;
         e->boxes[k].p = pflbm::make_params<float>(e->hps[k]);
+        // planes per CTA of the readback's analysis kernel (two CTAs per SM)
+        e->boxes[k].p.zchunk = pflbm::pick_zchunk(
+            int(((cfgs[k].nx + pflbm::TX - 1) / pflbm::TX) * ((cfgs[k].ny + pflbm::TY - 1) / pflbm::TY)),
+            int(cfgs[k].nz) - 2, e->sms, 2);
         e->boxes[k].f_off = f_off;
         e->boxes[k].n_off = n_off;
         f_off += uint64_t(e->q) * e->hps[k].N;
