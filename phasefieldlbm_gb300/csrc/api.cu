@@ -879,33 +879,36 @@ struct CkptHeader {
     uint64_t f_bytes, phi_bytes, avg_bytes;
 };
 
-int write_blob(std::ofstream &o, const void *dev, uint64_t bytes) {
+// `bytes` of device rows of `row` bytes, `pitch` bytes apart, to and from a
+// file without what pads them.
+int write_blob(std::ofstream &o, const void *dev, uint64_t bytes, size_t row, size_t pitch) {
     constexpr size_t kChunkBytes = size_t(1) << 26;
-    std::unique_ptr<char[]> h(new (std::nothrow) char[kChunkBytes]);
+    const size_t step = std::max<size_t>(1, kChunkBytes / row);  // rows at a time
+    std::unique_ptr<char[]> h(new (std::nothrow) char[step * row]);
     if (!h) return fail(PFLBM_ERR_OUT_OF_MEMORY, "checkpoint staging buffer");
-    for (uint64_t off = 0; off < bytes; off += kChunkBytes) {
-        const size_t n = size_t(std::min<uint64_t>(kChunkBytes, bytes - off));
-        cudaError_t e = cudaMemcpy(h.get(), static_cast<const char *>(dev) + off, n, cudaMemcpyDeviceToHost);
+    for (uint64_t r = 0, rows = bytes / row; r < rows; r += step) {
+        const size_t n = size_t(std::min<uint64_t>(step, rows - r));
+        cudaError_t e = cudaMemcpy2D(h.get(), row, static_cast<const char *>(dev) + r * pitch, pitch, row, n,
+                                     cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "checkpoint D2H");
-        o.write(h.get(), std::streamsize(n));
+        o.write(h.get(), std::streamsize(n * row));
         if (!o) return fail(PFLBM_ERR_IO, "checkpoint write failed");
     }
     return PFLBM_OK;
 }
 
-int read_blob(std::ifstream &in, void *dev0, void *dev1, uint64_t bytes) {
+int read_blob(std::ifstream &in, void *dev, uint64_t bytes, size_t row, size_t pitch) {
     constexpr size_t kChunkBytes = size_t(1) << 26;
-    std::unique_ptr<char[]> h(new (std::nothrow) char[kChunkBytes]);
+    const size_t step = std::max<size_t>(1, kChunkBytes / row);
+    std::unique_ptr<char[]> h(new (std::nothrow) char[step * row]);
     if (!h) return fail(PFLBM_ERR_OUT_OF_MEMORY, "checkpoint staging buffer");
-    for (uint64_t off = 0; off < bytes; off += kChunkBytes) {
-        const size_t n = size_t(std::min<uint64_t>(kChunkBytes, bytes - off));
-        in.read(h.get(), std::streamsize(n));
+    for (uint64_t r = 0, rows = bytes / row; r < rows; r += step) {
+        const size_t n = size_t(std::min<uint64_t>(step, rows - r));
+        in.read(h.get(), std::streamsize(n * row));
         if (!in) return fail(PFLBM_ERR_IO, "checkpoint truncated");
-        for (void *d : {dev0, dev1}) {
-            if (!d) continue;
-            cudaError_t e = cudaMemcpy(static_cast<char *>(d) + off, h.get(), n, cudaMemcpyHostToDevice);
-            if (e != cudaSuccess) return cuda_fail(e, "checkpoint H2D");
-        }
+        cudaError_t e = cudaMemcpy2D(static_cast<char *>(dev) + r * pitch, pitch, h.get(), row, row, n,
+                                     cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return cuda_fail(e, "checkpoint H2D");
     }
     return PFLBM_OK;
 }
@@ -930,11 +933,13 @@ int pflbm_save_checkpoint(pflbm_sim *s, const char *path) {
     std::ofstream o(path, std::ios::binary | std::ios::trunc);
     if (!o) return fail(PFLBM_ERR_IO, std::string("cannot open ") + path);
     o.write(reinterpret_cast<const char *>(&h), sizeof h);
-    int rc = write_blob(o, s->eng->f_ptr(s->parity), h.f_bytes);
-    if (!rc) rc = write_blob(o, s->eng->f_ptr(s->parity ^ 1), h.f_bytes);
-    if (!rc) rc = write_blob(o, s->eng->phi_ptr(s->parity), h.phi_bytes);
-    if (!rc) rc = write_blob(o, s->eng->phi_ptr(s->parity ^ 1), h.phi_bytes);
-    if (!rc && h.avg_bytes) rc = write_blob(o, s->eng->avg_ptr(), h.avg_bytes);
+    const size_t nx = s->hp.nx, sf = h.f_bytes / (s->hp.N * s->cfg.velocity_set), st = s->eng->real_bytes();
+    const size_t fp = s->eng->f_pitch(), pp = s->eng->phi_pitch();
+    int rc = write_blob(o, s->eng->f_ptr(s->parity), h.f_bytes, nx * sf, fp);
+    if (!rc) rc = write_blob(o, s->eng->f_ptr(s->parity ^ 1), h.f_bytes, nx * sf, fp);
+    if (!rc) rc = write_blob(o, s->eng->phi_ptr(s->parity), h.phi_bytes, nx * st, pp);
+    if (!rc) rc = write_blob(o, s->eng->phi_ptr(s->parity ^ 1), h.phi_bytes, nx * st, pp);
+    if (!rc && h.avg_bytes) rc = write_blob(o, s->eng->avg_ptr(), h.avg_bytes, nx * st, nx * st);
     return rc;
 }
 
@@ -953,11 +958,13 @@ int pflbm_load_checkpoint(pflbm_sim *s, const char *path) {
         h.phi_bytes != s->eng->phi_bytes() || h.avg_bytes != s->eng->avg_bytes())
         return fail(PFLBM_ERR_INVALID_ARG, "checkpoint does not match this simulation's grid, lattice or storage");
     cudaStreamSynchronize(s->stream);
-    int rc = read_blob(in, s->eng->f_ptr(0), nullptr, h.f_bytes);
-    if (!rc) rc = read_blob(in, s->eng->f_ptr(1), nullptr, h.f_bytes);
-    if (!rc) rc = read_blob(in, s->eng->phi_ptr(0), nullptr, h.phi_bytes);
-    if (!rc) rc = read_blob(in, s->eng->phi_ptr(1), nullptr, h.phi_bytes);
-    if (!rc && h.avg_bytes) rc = read_blob(in, s->eng->avg_ptr(), nullptr, h.avg_bytes);
+    const size_t nx = s->hp.nx, sf = h.f_bytes / (s->hp.N * s->cfg.velocity_set), st = s->eng->real_bytes();
+    const size_t fp = s->eng->f_pitch(), pp = s->eng->phi_pitch();
+    int rc = read_blob(in, s->eng->f_ptr(0), h.f_bytes, nx * sf, fp);
+    if (!rc) rc = read_blob(in, s->eng->f_ptr(1), h.f_bytes, nx * sf, fp);
+    if (!rc) rc = read_blob(in, s->eng->phi_ptr(0), h.phi_bytes, nx * st, pp);
+    if (!rc) rc = read_blob(in, s->eng->phi_ptr(1), h.phi_bytes, nx * st, pp);
+    if (!rc && h.avg_bytes) rc = read_blob(in, s->eng->avg_ptr(), h.avg_bytes, nx * st, nx * st);
     if (rc) return rc;
     s->eng->reset_counters(s->stream);
     s->eng->set_counter(0, h.step, s->stream);

@@ -60,6 +60,10 @@ class Engine {
     // Raw state buffers for checkpoints.
     virtual void *f_ptr(int k) = 0;
     virtual void *phi_ptr(int k) = 0;
+    // distance of consecutive rows of f and phi on the device, in bytes
+    virtual size_t f_pitch() const = 0;
+    virtual size_t phi_pitch() const = 0;
+    // bytes of the arrays without what pads their rows
     virtual uint64_t f_bytes() const = 0;
     virtual uint64_t phi_bytes() const = 0;
     virtual uint64_t avg_bytes() const = 0;

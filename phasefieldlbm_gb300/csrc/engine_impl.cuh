@@ -20,8 +20,9 @@ Params<T> make_params(const HostParams &h) {
     Params<T> p{};
     const bool f = sizeof(T) == 4;
     p.nx = h.nx; p.ny = h.ny; p.nz = h.nz;
+    p.px = h.nx;  // EngineT::allocate may pad the rows
     p.plane = h.nx * h.ny;
-    p.N = h.N;
+    p.N = p.Nd = h.N;
     p.zchunk = 1;  // set for a kernel by pick_zchunk
     // FP32 runs use the float-rounded constants exactly as the reference
     // computes them; FP64 runs use the double values.
@@ -50,13 +51,13 @@ Params<T> make_params(const HostParams &h) {
     return p;
 }
 
-// Tensor maps of the TMA collide kernel for one grid: f as (x, y, z, q) with
+// Tensor maps of the TMA collide kernel for one grid (rows px apart): f as (x, y, z, q) with
 // boxes (BWN, TY, 1, 1) for the c_x = 0 directions and (BWW, TY, 1, 1) for
 // the others, phi as (x, y, z) with boxes (PBW, PBH, 1). False when the
 // driver entry point is missing or the encoder rejects the layout.
 template <int QQ, class S, class L = TmaLayout<QQ, S>>
 bool encode_collide_maps(const S *f, const typename Store<S>::T *phi, uint64_t nx, uint64_t ny, uint64_t nz,
-                         CUtensorMap &fmapn, CUtensorMap &fmapw, CUtensorMap &phimap) {
+                         uint64_t px, CUtensorMap &fmapn, CUtensorMap &fmapw, CUtensorMap &phimap) {
     using T = typename Store<S>::T;
     using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -74,9 +75,9 @@ bool encode_collide_maps(const S *f, const typename Store<S>::T *phi, uint64_t n
                                    : std::is_same<S, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                                     : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const CUtensorMapDataType pt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    const uint64_t N = nx * ny * nz;
+    const uint64_t N = px * ny * nz;
     const cuuint64_t fdim[4] = {nx, ny, nz, cuuint64_t(QQ)};
-    const cuuint64_t fstr[3] = {nx * sizeof(S), nx * ny * sizeof(S), N * sizeof(S)};
+    const cuuint64_t fstr[3] = {px * sizeof(S), px * ny * sizeof(S), N * sizeof(S)};
     // boxes of the layout's tile: the TMA writes exactly what L's shared-memory
     // plan and transaction count expect
     const cuuint32_t fboxn[4] = {cuuint32_t(L::BWN), cuuint32_t(L::TY), 1, 1};
@@ -88,7 +89,7 @@ bool encode_collide_maps(const S *f, const typename Store<S>::T *phi, uint64_t n
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
     const cuuint64_t pdim[3] = {nx, ny, nz};
-    const cuuint64_t pstr[2] = {nx * sizeof(T), nx * ny * sizeof(T)};
+    const cuuint64_t pstr[2] = {px * sizeof(T), px * ny * sizeof(T)};
     const cuuint32_t pbox[3] = {cuuint32_t(L::PBW), cuuint32_t(L::PBH), 1};
     return enc(&phimap, pt, 3, const_cast<T *>(phi), pdim, pstr, pbox, one4, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -103,12 +104,39 @@ class EngineT final : public Engine {
     EngineT(const HostParams &h, uint32_t flags) : h_(h), flags_(flags) { p_ = make_params<T>(h); }
     ~EngineT() override { free_all(); }
 
+    // Rows that do not start on 16-byte boundaries are padded, so that every
+    // grid runs the TMA-fed collide and the float4 phase step (D3Q27 FP32
+    // 101x93x251: collide 205 -> 147 us, phase 55 -> 20 us against the
+    // plain-load kernels).
+    // Where the padded arrays do not fit, the grid keeps its own rows and the
+    // plain-load kernels.
     int allocate(std::string &err) override {
-        const uint64_t N = h_.N, plane = uint64_t(h_.nx) * h_.ny;
+        const uint32_t unit = 32 / sizeof(S);  // 32-byte sectors
+        const bool aligned = (uint64_t(h_.nx) * sizeof(S)) % 16 == 0 && (uint64_t(h_.nx) * sizeof(T)) % 16 == 0;
+        const char *no_tma = std::getenv("PFLBM_NO_TMA");
+        const uint32_t padded = (h_.nx + unit - 1) / unit * unit;
+        int rc = PFLBM_ERR_OUT_OF_MEMORY;
+        if (!aligned && !(no_tma && no_tma[0] == '1') &&
+            uint64_t(padded) * h_.ny * h_.nz < (uint64_t(1) << 32))  // 32-bit node indices
+            rc = allocate_rows(padded, err);
+        if (rc == PFLBM_ERR_OUT_OF_MEMORY) rc = allocate_rows(h_.nx, err);
+        if (rc) return rc;
+        if (cudaDeviceSynchronize() != cudaSuccess) {
+            err = cudaGetErrorString(cudaGetLastError());
+            return PFLBM_ERR_CUDA;
+        }
+        setup_tma();
+        choose_zchunk();
+        return PFLBM_OK;
+    }
+
+    int allocate_rows(uint32_t px, std::string &err) {
+        const uint64_t Nd = h_.N, plane = uint64_t(px) * h_.ny, N = plane * h_.nz;
         struct Req {
             void **ptr;
             size_t bytes;
         };
+        const bool averages = flags_ & (PFLBM_FLAG_TIME_AVERAGE | PFLBM_FLAG_REYNOLDS_MOMENTS);
         Req reqs[] = {
             {reinterpret_cast<void **>(&f_[0]), sizeof(S) * QQ * N},
             {reinterpret_cast<void **>(&f_[1]), sizeof(S) * QQ * N},
@@ -116,17 +144,17 @@ class EngineT final : public Engine {
             {reinterpret_cast<void **>(&phi_[1]), sizeof(T) * N},
             {reinterpret_cast<void **>(&j_), sizeof(T) * 3 * N},
             {reinterpret_cast<void **>(&top_), sizeof(T) * 22 * plane},
-            {reinterpret_cast<void **>(&macro_), sizeof(T) * M_COUNT * N},
+            {reinterpret_cast<void **>(&macro_), sizeof(T) * M_COUNT * Nd},
             {reinterpret_cast<void **>(&counters_), sizeof(unsigned long long) * 2},
             {reinterpret_cast<void **>(&err_), sizeof(unsigned int) * 4},
             {reinterpret_cast<void **>(&partial_), sizeof(double) * RED_FIELDS * kRedBlocks},
+            {reinterpret_cast<void **>(&avg_), averages ? sizeof(T) * 10 * Nd : 0},
+            {reinterpret_cast<void **>(&vort_), flags_ & PFLBM_FLAG_VORTICITY ? sizeof(T) * 4 * Nd : 0},
         };
         // fault injection on the host: PFLBM_ALLOC_LIMIT_BYTES caps the
         // device bytes one simulation may take (allocation fails cleanly)
         uint64_t planned = 0;
         for (auto &r : reqs) planned += r.bytes;
-        if (flags_ & (PFLBM_FLAG_TIME_AVERAGE | PFLBM_FLAG_REYNOLDS_MOMENTS)) planned += sizeof(T) * 10 * N;
-        if (flags_ & PFLBM_FLAG_VORTICITY) planned += sizeof(T) * 4 * N;
         if (const char *lim = std::getenv("PFLBM_ALLOC_LIMIT_BYTES")) {
             const unsigned long long cap = std::strtoull(lim, nullptr, 10);
             if (cap > 0 && planned > cap) {
@@ -136,6 +164,7 @@ class EngineT final : public Engine {
             }
         }
         for (auto &r : reqs) {
+            if (r.bytes == 0) continue;
             if (cudaMalloc(r.ptr, r.bytes) != cudaSuccess) {
                 cudaGetLastError();
                 err = "cudaMalloc failed (" + std::to_string(r.bytes) + " bytes)";
@@ -145,32 +174,9 @@ class EngineT final : public Engine {
             cudaMemset(*r.ptr, 0, r.bytes);
             bytes_ += r.bytes;
         }
-        if (flags_ & (PFLBM_FLAG_TIME_AVERAGE | PFLBM_FLAG_REYNOLDS_MOMENTS)) {
-            if (cudaMalloc(&avg_, sizeof(T) * 10 * N) != cudaSuccess) {
-                cudaGetLastError();
-                err = "cudaMalloc failed (averages)";
-                free_all();
-                return PFLBM_ERR_OUT_OF_MEMORY;
-            }
-            cudaMemset(avg_, 0, sizeof(T) * 10 * N);
-            bytes_ += sizeof(T) * 10 * N;
-        }
-        if (flags_ & PFLBM_FLAG_VORTICITY) {
-            if (cudaMalloc(&vort_, sizeof(T) * 4 * N) != cudaSuccess) {
-                cudaGetLastError();
-                err = "cudaMalloc failed (vorticity)";
-                free_all();
-                return PFLBM_ERR_OUT_OF_MEMORY;
-            }
-            cudaMemset(vort_, 0, sizeof(T) * 4 * N);
-            bytes_ += sizeof(T) * 4 * N;
-        }
-        if (cudaDeviceSynchronize() != cudaSuccess) {
-            err = cudaGetErrorString(cudaGetLastError());
-            return PFLBM_ERR_CUDA;
-        }
-        setup_tma();
-        choose_zchunk();
+        p_.px = px;
+        p_.plane = uint32_t(plane);
+        p_.N = N;
         return PFLBM_OK;
     }
 
@@ -225,10 +231,10 @@ class EngineT final : public Engine {
         if (const char *e = std::getenv("PFLBM_NO_VEC")) no_vec_ = e[0] == '1';
         if (const char *e = std::getenv("PFLBM_NO_TMA"))
             if (e[0] == '1') return;
-        if ((uint64_t(h_.nx) * sizeof(S)) % 16 != 0 || (uint64_t(h_.nx) * sizeof(T)) % 16 != 0) return;
+        if ((uint64_t(p_.px) * sizeof(S)) % 16 != 0 || (uint64_t(p_.px) * sizeof(T)) % 16 != 0) return;
         using L = TmaLayout<QQ, S>;
         for (int k = 0; k < 2; ++k)
-            if (!encode_collide_maps<QQ, S>(f_[k], phi_[k], h_.nx, h_.ny, h_.nz, fmapn_[k], fmapw_[k], phimap_[k]))
+            if (!encode_collide_maps<QQ, S>(f_[k], phi_[k], h_.nx, h_.ny, h_.nz, p_.px, fmapn_[k], fmapw_[k], phimap_[k]))
                 return;
         if (cudaFuncSetAttribute(k_collide_tma<QQ, JET, S, MODE_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(L::total)) != cudaSuccess ||
@@ -253,13 +259,15 @@ class EngineT final : public Engine {
         // step of 16-bit D3Q19 storage, whose collide is issue-bound (FP32
         // and D3Q27 stay faster with one node per thread and twice the
         // warps). PFLBM_NO_PAIR=1 keeps one node per thread; PFLBM_PAIR=1
-        // selects the pair kernel for every FP32/16-bit lattice (tests).
+        // selects the pair kernel for every FP32/16-bit lattice (tests). Grids
+        // with padded rows keep one node per thread: their results were always
+        // those of the one-node kernels.
         use_pair_ = false;
         if constexpr (sizeof(T) == 4) {
             const char *no = std::getenv("PFLBM_NO_PAIR");
             const char *force = std::getenv("PFLBM_PAIR");
             const bool want = (force && force[0] == '1') || (sizeof(S) == 2 && QQ == 19);
-            if (want && !(no && no[0] == '1') && h_.nx % 2 == 0) {
+            if (want && !(no && no[0] == '1') && p_.px == h_.nx) {
                 if (cudaFuncSetAttribute(k_collide_pair<QQ, JET, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          int(PairLayout<QQ, S>::total)) == cudaSuccess)
                     use_pair_ = true;
@@ -350,8 +358,8 @@ class EngineT final : public Engine {
         if (ev) cudaEventRecord(ev[1], s);
         if (ev) cudaEventRecord(ev[2], s);
         if constexpr (std::is_same<T, float>::value) {
-            if (h_.nx % 4 == 0 && !no_vec_) {
-                const dim3 g4((h_.nx / 4 + 31) / 32, (h_.ny + 7) / 8, JET ? h_.nz + 4 : h_.nz);
+            if (p_.px % 4 == 0 && !no_vec_) {
+                const dim3 g4(((h_.nx + 3) / 4 + 31) / 32, (h_.ny + 7) / 8, JET ? h_.nz + 4 : h_.nz);
                 k_phase_v4<QQ, JET, S><<<g4, node_block(), 0, s>>>(p_, b);
             } else {
                 k_phase<QQ, JET, S><<<node_grid(), node_block(), 0, s>>>(p_, b);
@@ -405,6 +413,8 @@ class EngineT final : public Engine {
     unsigned int *error_word() override { return err_; }
     void *f_ptr(int k) override { return f_[k]; }
     void *phi_ptr(int k) override { return phi_[k]; }
+    size_t f_pitch() const override { return sizeof(S) * p_.px; }
+    size_t phi_pitch() const override { return sizeof(T) * p_.px; }
     uint64_t f_bytes() const override { return sizeof(S) * QQ * h_.N; }
     uint64_t phi_bytes() const override { return sizeof(T) * h_.N; }
     uint64_t avg_bytes() const override { return avg_ ? sizeof(T) * 10 * h_.N : 0; }

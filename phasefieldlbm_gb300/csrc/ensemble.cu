@@ -359,7 +359,7 @@ class Ensemble {
             for (size_t k = 0; k < boxes.size(); ++k) {
                 const BoxDev &bx = boxes[k];
                 if (!encode_collide_maps<QQ, float, BatchLayout<QQ, G>>(bp.f[par] + bx.f_off, bp.phi[par] + bx.n_off,
-                                                                        bx.p.nx, bx.p.ny, bx.p.nz, m.fn[k], m.fw[k],
+                                                                        bx.p.nx, bx.p.ny, bx.p.nz, bx.p.px, m.fn[k], m.fw[k],
                                                                         m.phi[k]))
                     return false;
             }

@@ -28,7 +28,7 @@ struct InitGeom {
 template <class T>
 __global__ void k_init_fields(const Params<T> p, const InitGeom g, T *macro) {
     const int nx = p.nx, ny = p.ny, nz = p.nz;
-    const uint64_t N = p.N;
+    const uint64_t N = p.Nd;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z * blockDim.z + threadIdx.z;
@@ -65,25 +65,26 @@ __global__ void k_init_distros(const Params<typename Store<S>::T> p, S *fa, S *f
                                typename Store<S>::T *phib, const typename Store<S>::T *macro) {
     using T = typename Store<S>::T;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
-    const uint64_t N = p.N;
+    const uint64_t N = p.N, Nd = p.Nd;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z * blockDim.z + threadIdx.z;
     if (x >= nx || y >= ny || z >= nz) return;
     const uint64_t i = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * (y + static_cast<uint64_t>(ny) * z);
-    const T phi0 = macro[M_PHI * N + i];
+    const uint64_t ip = static_cast<uint64_t>(x) + static_cast<uint64_t>(p.px) * (y + static_cast<uint64_t>(ny) * z);
+    const T phi0 = macro[M_PHI * Nd + i];
     if (x < 1 || x > nx - 2 || y < 1 || y > ny - 2 || z < 1 || z > nz - 2) {
-        phia[i] = phi0;
-        phib[i] = phi0;
+        phia[ip] = phi0;
+        phib[ip] = phi0;
         return;
     }
-    const T rho = macro[M_RHO * N + i], ux = macro[M_UX * N + i], uy = macro[M_UY * N + i], uz = macro[M_UZ * N + i];
+    const T rho = macro[M_RHO * Nd + i], ux = macro[M_UX * Nd + i], uy = macro[M_UY * Nd + i], uz = macro[M_UZ * Nd + i];
 #pragma unroll
     for (int q = 0; q < QQ; ++q) {
         const T v = feq_q<QQ, T>(q, rho, ux, uy, uz);
-        const int64_t off = kCX[q] + static_cast<int64_t>(kCY[q]) * nx + static_cast<int64_t>(kCZ[q]) * static_cast<int64_t>(p.plane);
-        Store<S>::store(fa, q * N + i - off, v, static_cast<T>(1.0 / weight<QQ>(q)));
-        Store<S>::store(fb, q * N + i - off, v, static_cast<T>(1.0 / weight<QQ>(q)));
+        const int64_t off = kCX[q] + static_cast<int64_t>(kCY[q]) * p.px + static_cast<int64_t>(kCZ[q]) * static_cast<int64_t>(p.plane);
+        Store<S>::store(fa, q * N + ip - off, v, static_cast<T>(1.0 / weight<QQ>(q)));
+        Store<S>::store(fb, q * N + ip - off, v, static_cast<T>(1.0 / weight<QQ>(q)));
     }
     T s = T(0);
 #pragma unroll
@@ -91,8 +92,8 @@ __global__ void k_init_distros(const Params<typename Store<S>::T> p, S *fa, S *f
         const T w = static_cast<T>(weight7(q));
         s += w * phi0 * (T(1) + T(4) * cdot<T>(kCX[q], kCY[q], kCZ[q], ux, uy, uz));
     }
-    phia[i] = s;
-    phib[i] = phi0;
+    phia[ip] = s;
+    phib[ip] = phi0;
 }
 
 // Ghost-shell values of the reference's arrays after a step (analysis):
@@ -101,7 +102,7 @@ __global__ void k_init_distros(const Params<typename Store<S>::T> p, S *fa, S *f
 template <class T>
 __global__ void k_analysis_ghosts(const Params<T> p, int jet, uint32_t t, T *macro) {
     const int nx = p.nx, ny = p.ny, nz = p.nz;
-    const uint64_t N = p.N;
+    const uint64_t N = p.Nd;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z * blockDim.z + threadIdx.z;
@@ -119,7 +120,7 @@ __global__ void k_analysis_ghosts(const Params<T> p, int jet, uint32_t t, T *mac
         macro[M_UY * N + i] = uy;
         macro[M_UZ * N + i] = uz;
     } else if (z == nz - 1 && x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2) {
-        const uint64_t j = i - p.plane;
+        const uint64_t j = i - static_cast<uint64_t>(nx) * ny;
         for (int s : {(int)M_RHO, (int)M_PHI, (int)M_UX, (int)M_UY, (int)M_UZ}) macro[s * N + i] = macro[s * N + j];
     }
 }
@@ -128,7 +129,7 @@ __global__ void k_analysis_ghosts(const Params<T> p, int jet, uint32_t t, T *mac
 template <class T>
 __global__ void k_vorticity(const Params<T> p, const T *macro, T *vort) {
     const int nx = p.nx, ny = p.ny, nz = p.nz;
-    const uint64_t N = p.N;
+    const uint64_t N = p.Nd;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z * blockDim.z + threadIdx.z;
@@ -137,7 +138,7 @@ __global__ void k_vorticity(const Params<T> p, const T *macro, T *vort) {
     T wx = T(0), wy = T(0), wz = T(0);
     if (x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && z < nz - 1) {
         const T *ux = macro + M_UX * N, *uy = macro + M_UY * N, *uz = macro + M_UZ * N;
-        const uint64_t sx = 1, sy = nx, sz = p.plane;
+        const uint64_t sx = 1, sy = nx, sz = static_cast<uint64_t>(nx) * ny;
         const T h = T(0.5);
         const T duz_dy = h * (uz[i + sy] - uz[i - sy]);
         const T duy_dz = h * (uy[i + sz] - uy[i - sz]);
@@ -162,7 +163,7 @@ constexpr int RED_THREADS = 256;
 template <class T>
 __global__ void __launch_bounds__(RED_THREADS) k_reduce_partial(const Params<T> p, const T *macro, double *partial) {
     const int nx = p.nx, ny = p.ny, nz = p.nz;
-    const uint64_t N = p.N;
+    const uint64_t N = p.Nd;
     const uint64_t nint = static_cast<uint64_t>(nx - 2) * (ny - 2) * (nz - 2);
     double acc[RED_FIELDS] = {0};
     for (uint64_t k = blockIdx.x * static_cast<uint64_t>(RED_THREADS) + threadIdx.x; k < nint;

@@ -20,7 +20,7 @@
 //               outflow rebuilds and the outflow ghost-plane copy.
 //
 // Data layout in HBM (SoA, x fastest, ghost shell included as in the
-// reference): f[q][z][y][x] twice (ping-pong), phi[z][y][x] twice, the
+// reference, rows Params::px apart): f[q][z][y][x] twice (ping-pong), phi[z][y][x] twice, the
 // phase flux J[3][z][y][x], and for the jet 13 moments of plane nz-2 and
 // 9 of plane 1 for the outflow and inflow rebuilds done by k_phase.
 //
@@ -77,17 +77,19 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const uint64_t N = p.N, plane = p.plane;
     // node index, 32-bit (N < 2^32 is checked on the host)
-    const uint32_t node = uint32_t(x) + uint32_t(nx) * (uint32_t(y) + uint32_t(ny) * uint32_t(z));
+    const uint32_t node = uint32_t(x) + p.px * (uint32_t(y) + uint32_t(ny) * uint32_t(z));
     const uint64_t base = node;
+    // the same node in the arrays with rows of nx
+    const uint64_t Nd = p.Nd, dense = uint32_t(x) + uint32_t(nx) * (uint32_t(y) + uint32_t(ny) * uint32_t(z));
     // running averages of this node, loaded before any store of the node
     // (the compiler cannot move them above the population stores, which it
     // cannot prove do not alias them), so their latency overlaps the
     // collision instead of following it
     T av_old[10];
     if constexpr (mode_average(MODE)) {
-        if (active && PFLBM_GUARD(base < N, b.err)) {
+        if (active && PFLBM_GUARD(dense < Nd, b.err)) {
 #pragma unroll
-            for (int k = 0; k < 10; ++k) av_old[k] = b.avg[k * N + base];
+            for (int k = 0; k < 10; ++k) av_old[k] = b.avg[k * Nd + dense];
         }
     }
     const T st = -p.sigma * curvature * ind;
@@ -127,24 +129,24 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
 
     if constexpr (MODE == MODE_ANALYSIS) {
         T *mc = b.macro;
-        mc[M_RHO * N + base] = m.rho;
-        mc[M_UX * N + base] = m.ux;
-        mc[M_UY * N + base] = m.uy;
-        mc[M_UZ * N + base] = m.uz;
-        mc[M_PXX * N + base] = m.pxx;
-        mc[M_PYY * N + base] = m.pyy;
-        mc[M_PZZ * N + base] = m.pzz;
-        mc[M_PXY * N + base] = m.pxy;
-        mc[M_PXZ * N + base] = m.pxz;
-        mc[M_PYZ * N + base] = m.pyz;
-        mc[M_PHI * N + base] = phi;
-        mc[M_NX * N + base] = n_x;
-        mc[M_NY * N + base] = n_y;
-        mc[M_NZ * N + base] = n_z;
-        mc[M_IND * N + base] = ind;
-        mc[M_FX * N + base] = fx;
-        mc[M_FY * N + base] = fy;
-        mc[M_FZ * N + base] = fz;
+        mc[M_RHO * Nd + dense] = m.rho;
+        mc[M_UX * Nd + dense] = m.ux;
+        mc[M_UY * Nd + dense] = m.uy;
+        mc[M_UZ * Nd + dense] = m.uz;
+        mc[M_PXX * Nd + dense] = m.pxx;
+        mc[M_PYY * Nd + dense] = m.pyy;
+        mc[M_PZZ * Nd + dense] = m.pzz;
+        mc[M_PXY * Nd + dense] = m.pxy;
+        mc[M_PXZ * Nd + dense] = m.pxz;
+        mc[M_PYZ * Nd + dense] = m.pyz;
+        mc[M_PHI * Nd + dense] = phi;
+        mc[M_NX * Nd + dense] = n_x;
+        mc[M_NY * Nd + dense] = n_y;
+        mc[M_NZ * Nd + dense] = n_z;
+        mc[M_IND * Nd + dense] = ind;
+        mc[M_FX * Nd + dense] = fx;
+        mc[M_FY * Nd + dense] = fy;
+        mc[M_FZ * Nd + dense] = fz;
         return;
     } else {
         // periodic-edge store offsets: P = wrap(S + c) - c. Node indices
@@ -153,8 +155,8 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
         // back into [0, N) exactly.
         const uint32_t ex_p = (x == nx - 2) ? 0u - uint32_t(nx - 2) : 0u;  // cx = +1
         const uint32_t ex_m = (x == 1) ? uint32_t(nx - 2) : 0u;            // cx = -1
-        const uint32_t ey_p = (y == ny - 2) ? 0u - uint32_t(ny - 2) * uint32_t(nx) : 0u;
-        const uint32_t ey_m = (y == 1) ? uint32_t(ny - 2) * uint32_t(nx) : 0u;
+        const uint32_t ey_p = (y == ny - 2) ? 0u - uint32_t(ny - 2) * p.px : 0u;
+        const uint32_t ey_m = (y == 1) ? uint32_t(ny - 2) * p.px : 0u;
         uint32_t ez_p = 0u, ez_m = 0u;
         if constexpr (!JET) {
             ez_p = (z == nz - 2) ? 0u - uint32_t(nz - 2) * uint32_t(plane) : 0u;
@@ -175,8 +177,8 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
         // (sround.cuh), with the bits of this node's half of its pair.
         constexpr bool kSR = std::is_same<S, __nv_bfloat16>::value;
         uint32_t sr_seed = 0u;
-        if constexpr (kSR) sr_seed = sr_pair_seed(node >> 1, t);
-        const uint32_t sr_shift = (node & 1u) ? 16u : 0u;
+        if constexpr (kSR) sr_seed = sr_pair_seed(uint32_t(dense) >> 1, t);
+        const uint32_t sr_shift = (dense & 1u) ? 16u : 0u;
         auto put = [&](int q, uint32_t idx, T v) {
             const T inv_w = static_cast<T>(1.0 / weight<QQ>(q));
             if constexpr (kSR) {
@@ -209,7 +211,7 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
         if constexpr (JET) {
             if (z == nz - 2) {
                 // moments of the last fluid plane for the outflow rebuild
-                const uint64_t c2 = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * y;
+                const uint64_t c2 = static_cast<uint64_t>(x) + static_cast<uint64_t>(p.px) * y;
                 if (!PFLBM_GUARD(c2 < plane, b.err)) return;
                 T *tp = b.top;
                 tp[0 * plane + c2] = m.rho;
@@ -228,7 +230,7 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
             }
             if (z == 1) {
                 // moments of the first fluid plane for the inflow rebuild
-                const uint64_t c2 = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * y;
+                const uint64_t c2 = static_cast<uint64_t>(x) + static_cast<uint64_t>(p.px) * y;
                 if (!PFLBM_GUARD(c2 < plane, b.err)) return;
                 T *bp = b.top + 13 * plane;
                 bp[0 * plane + c2] = m.ux;
@@ -247,14 +249,14 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
             const T tf = static_cast<T>(t + 1u);
             T *av = b.avg;
             auto upd = [&](int slot, uint64_t i, T nv_) {
-                if (!PFLBM_GUARD(i < N, b.err)) return;
-                const T o = av[slot * N + i];
-                av[slot * N + i] = o + (nv_ - o) / tf;
+                if (!PFLBM_GUARD(i < Nd, b.err)) return;
+                const T o = av[slot * Nd + i];
+                av[slot * Nd + i] = o + (nv_ - o) / tf;
             };
             const T now[10] = {phi, m.ux, m.uy, m.uz, m.ux * m.ux, m.uy * m.uy, m.uz * m.uz,
                                m.ux * m.uy, m.ux * m.uz, m.uy * m.uz};
 #pragma unroll
-            for (int k = 0; k < 10; ++k) av[k * N + base] = av_old[k] + (now[k] - av_old[k]) / tf;
+            for (int k = 0; k < 10; ++k) av[k * Nd + dense] = av_old[k] + (now[k] - av_old[k]) / tf;
             if constexpr (JET) {
                 if (z == 1 && in_disc<T>(p, x, y)) {
                     // ghost inlet node (x,y,0) holds phi = 1 and the inlet velocity
@@ -309,7 +311,7 @@ __device__ __forceinline__ void collide_tile(const Params<typename Store<S>::T> 
             const int gx = x0 - 2 + lx, gy = y0 - 2 + ly;
             T v = T(0);
             if (gx >= 0 && gx < nx && gy >= 0 && gy < ny && zp >= 0 && zp < nz)
-                v = b.phi_src[gx + static_cast<uint64_t>(nx) * (gy + static_cast<uint64_t>(ny) * zp)];
+                v = b.phi_src[gx + static_cast<uint64_t>(p.px) * (gy + static_cast<uint64_t>(ny) * zp)];
             s_phi[slot][ly][lx] = v;
         }
     };
@@ -352,11 +354,11 @@ __device__ __forceinline__ void collide_tile(const Params<typename Store<S>::T> 
         // issue the pull loads of this node first; they land while the
         // stencil work below runs
         T pop[QQ];
-        const uint64_t base = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * (y + static_cast<uint64_t>(ny) * z);
+        const uint64_t base = static_cast<uint64_t>(x) + static_cast<uint64_t>(p.px) * (y + static_cast<uint64_t>(ny) * z);
         if (col) {
 #pragma unroll
             for (int q = 0; q < QQ; ++q) {
-                const int64_t off = kCX[q] + static_cast<int64_t>(kCY[q]) * nx + static_cast<int64_t>(kCZ[q]) * static_cast<int64_t>(plane);
+                const int64_t off = kCX[q] + static_cast<int64_t>(kCY[q]) * p.px + static_cast<int64_t>(kCZ[q]) * static_cast<int64_t>(plane);
                 pop[q] = Store<S>::load(b.f_src, q * N + base - off, static_cast<T>(weight<QQ>(q)));
             }
         } else if constexpr (mode_closure(MODE) && std::is_same<T, float>::value) {

@@ -300,7 +300,7 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
             const int gx = x0 - L::PXO + lx, gy = y0 - 2 + ly;
             T v = T(0);
             if (gx >= 0 && gx < nx && gy >= 0 && gy < ny && zp >= 0 && zp < nz)
-                v = b.phi_src[gx + static_cast<uint64_t>(nx) * (gy + static_cast<uint64_t>(ny) * zp)];
+                v = b.phi_src[gx + static_cast<uint64_t>(p.px) * (gy + static_cast<uint64_t>(ny) * zp)];
             phi_at(slot, ly, lx) = v;
         }
     }

@@ -12,8 +12,8 @@ namespace pflbm {
 template <class T>
 struct Params {
     uint32_t nx, ny, nz;
-    uint32_t plane;  // nx*ny
-    uint64_t N;      // nx*ny*nz
+    uint32_t plane;  // px*ny
+    uint64_t N;      // px*ny*nz
     int32_t zchunk;  // interior planes per CTA of the collide kernel
     T sigma, gamma, u_inf;
     T omega_ref;  // droplet (globalFunctions.cuh:426-429)
@@ -27,6 +27,13 @@ struct Params {
     int32_t noise_mode;
     uint32_t seed;
     float u_inf_f;
+    // f, phi, J and the boundary planes: rows px >= nx elements apart, so that
+    // every row starts on a 16-byte boundary whatever nx is (px == nx where it
+    // does anyway). The arrays a caller sees (macroscopic fields, averages,
+    // vorticity) have rows of nx. (Kept behind the others: which multiply-adds
+    // the compiler contracts depends on where the constants lie.)
+    uint32_t px;
+    uint64_t Nd;  // nx*ny*nz
 };
 
 // Storage of the shifted populations f' = f - w (the reference's f_eq is
@@ -88,8 +95,8 @@ struct StepBuffers {
     const unsigned long long *step_in;
     unsigned long long *step_out;
     uint32_t t_fixed;  // step index used when step_in is null (analysis)
-    T *avg;            // 10*N derived averages (or null)
-    T *macro;          // 18*N analysis output (or null)
+    T *avg;            // 10*Nd derived averages (or null)
+    T *macro;          // 18*Nd analysis output (or null)
     unsigned int *err; // device error flag
     const float *mlp;  // closure network blob (MODE_STEP_CLOSURE)
 };

@@ -20,10 +20,11 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
                                            uint32_t t) {
     using T = typename Store<S>::T;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
+    const uint64_t px = p.px;
     const uint64_t N = p.N, plane = p.plane;
-    const uint64_t X = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * (y + static_cast<uint64_t>(ny) * z);
+    const uint64_t X = static_cast<uint64_t>(x) + px * (y + static_cast<uint64_t>(ny) * z);
     auto idx = [&](int xx, int yy, int zz) -> uint64_t {
-        return static_cast<uint64_t>(xx) + static_cast<uint64_t>(nx) * (yy + static_cast<uint64_t>(ny) * zz);
+        return static_cast<uint64_t>(xx) + px * (yy + static_cast<uint64_t>(ny) * zz);
     };
     const T *phi = b.phi_src;
     const T *J = b.jflux;
@@ -56,7 +57,7 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
     }
     if (JET && z == nz - 2) {
         // BoundaryConditions.cuh:168 with the node's own phi and uz
-        const T uz = b.top[3 * plane + static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * y];
+        const T uz = b.top[3 * plane + static_cast<uint64_t>(x) + px * y];
         g6 = w1 * phiX * (T(1) - T(4) * uz);
     } else {
         const uint64_t s6 = idx(x, y, zp);
@@ -72,7 +73,7 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
             // entering (x,y,1) from a ghost column (x-cx, y-cy, 0) inside the
             // inlet disc get feq of the inlet state plus the regularised
             // non-equilibrium of this node's step-n moments.
-            const uint64_t cX = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * y;
+            const uint64_t cX = static_cast<uint64_t>(x) + px * y;
             const T *bp = b.top + 13 * plane;
             Macro<T> mX;
             mX.rho = T(1);
@@ -88,8 +89,8 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
                         T bux, buy, buz;
                         inflow_velocity<T>(p, gx, gy, t, bux, buy, buz);
                         const T v = feq_q<QQ, T>(q, T(1), bux, buy, buz) + p.omco_zmin * fneq_q<QQ, T>(q, kX);
-                        if (PFLBM_GUARD(static_cast<uint64_t>(gx) + static_cast<uint64_t>(nx) * gy < plane, b.err))
-                        Store<S>::store(b.f_dst, q * N + static_cast<uint64_t>(gx) + static_cast<uint64_t>(nx) * gy, v,
+                        if (PFLBM_GUARD(static_cast<uint64_t>(gx) + px * gy < plane, b.err))
+                        Store<S>::store(b.f_dst, q * N + static_cast<uint64_t>(gx) + px * gy, v,
                                         static_cast<T>(1.0 / weight<QQ>(q)));
                     }
                 }
@@ -103,7 +104,7 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
             // the ghost plane: equilibrium of the in-plane source column
             // (x-cx, y-cy), non-equilibrium and force of this node.
             const T *tp = b.top;
-            const uint64_t cX = static_cast<uint64_t>(x) + static_cast<uint64_t>(nx) * y;
+            const uint64_t cX = static_cast<uint64_t>(x) + px * y;
             Macro<T> mX;
             mX.rho = tp[cX];
             mX.ux = tp[plane + cX]; mX.uy = tp[2 * plane + cX]; mX.uz = tp[3 * plane + cX];
@@ -115,7 +116,7 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
             for (int q = 1; q < QQ; ++q) {
                 if (kCZ[q] == -1) {
                     const int bx = wrapi(x - kCX[q], nx), by = wrapi(y - kCY[q], ny);
-                    const uint64_t cb = static_cast<uint64_t>(bx) + static_cast<uint64_t>(nx) * by;
+                    const uint64_t cb = static_cast<uint64_t>(bx) + px * by;
                     const T rb = tp[cb], uxb = tp[plane + cb], uyb = tp[2 * plane + cb], uzb = tp[3 * plane + cb];
                     const T phib = phi[cb + plane * static_cast<uint64_t>(nz - 2)];
                     const T visc_local = (T(1) - phib) * p.visc_water + phib * p.visc_oil;
@@ -123,7 +124,7 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
                     const T v = feq_q<QQ, T>(q, rb, uxb, uyb, uzb) + omco * fneq_q<QQ, T>(q, kX) +
                                 T(0.5) * force_q<QQ, T>(q, uxb, uyb, uzb, fxX, fyX, fzX);
                     const uint64_t dst = q * N + static_cast<uint64_t>(x - kCX[q]) +
-                                         static_cast<uint64_t>(nx) * (static_cast<uint64_t>(y - kCY[q]) + static_cast<uint64_t>(ny) * (nz - 1));
+                                         px * (static_cast<uint64_t>(y - kCY[q]) + static_cast<uint64_t>(ny) * (nz - 1));
                     if (PFLBM_GUARD(dst < uint64_t(QQ) * N, b.err))
                         Store<S>::store(b.f_dst, dst, v, static_cast<T>(1.0 / weight<QQ>(q)));
                 }
@@ -155,7 +156,7 @@ __device__ __noinline__ void phase_node_outlined(const Params<float> &p, const S
 }
 
 // The phase sum of the 4 consecutive nodes x4 .. x4+3 of row (y, z), an
-// interior row of a grid with nx % 4 == 0 (shared by k_phase_v4 and the
+// interior row of a grid with px % 4 == 0 (shared by k_phase_v4 and the
 // ensemble's batch phase kernel).
 template <bool JET, class S>
 __device__ __forceinline__ void phase_vec4(const Params<float> &p, const StepBuffers<S, float> &b, int x4, int y,
@@ -164,7 +165,7 @@ __device__ __forceinline__ void phase_vec4(const Params<float> &p, const StepBuf
     const uint64_t N = p.N;
     const int ym = wrapi(y - 1, ny), yp = wrapi(y + 1, ny);
     const int zm = JET ? z - 1 : wrapi(z - 1, nz), zp = JET ? z + 1 : wrapi(z + 1, nz);
-    auto row = [&](int yy, int zz) -> uint64_t { return static_cast<uint64_t>(nx) * (yy + static_cast<uint64_t>(ny) * zz); };
+    auto row = [&](int yy, int zz) -> uint64_t { return static_cast<uint64_t>(p.px) * (yy + static_cast<uint64_t>(ny) * zz); };
     const float *phi = b.phi_src;
     const float *Jx = b.jflux, *Jy = b.jflux + N, *Jz = b.jflux + 2 * N;
     const uint64_t r0 = row(y, z);
@@ -215,13 +216,16 @@ __device__ __forceinline__ void phase_vec4(const Params<float> &p, const StepBuf
     // memory system completes with a read of the old sector (0.045 -> 0.043
     // ms on the 128x128x512 jet)
     if (!PFLBM_GUARD(r0 + x4 + 3 < N, b.err)) return;
-    if (x4 == 0) out[0] = pc.x;
-    if (x4 + 3 == nx - 1) out[3] = pc.w;
+    // (x >= nx - 1: the last ghost column and what pads the row)
+    if (x4 == 0 || x4 >= nx - 1) out[0] = pc.x;
+    if (x4 + 1 >= nx - 1) out[1] = pc.y;
+    if (x4 + 2 >= nx - 1) out[2] = pc.z;
+    if (x4 + 3 >= nx - 1) out[3] = pc.w;
     *reinterpret_cast<float4 *>(b.phi_dst + r0 + x4) = make_float4(out[0], out[1], out[2], out[3]);
 }
 
 // FP32 phase step with 128-bit accesses: one thread owns 4 consecutive x
-// nodes (nx % 4 == 0), reads the phi/J rows of its y and z neighbours as
+// nodes (px % 4 == 0), reads the phi/J rows of its y and z neighbours as
 // float4 and the two x-end neighbours (periodically wrapped) as scalars.
 // The jet's boundary planes z = 1 and nz-2 go through phase_node, one node
 // per thread, in grid slices of their own.
