@@ -404,7 +404,7 @@ class EngineT final : public Engine {
     }
     void enqueue_reduce(cudaStream_t s, double *dev_out) override {
         k_reduce_partial<T><<<kRedBlocks, RED_THREADS, 0, s>>>(p_, macro_, partial_);
-        k_reduce_final<<<1, 32, 0, s>>>(partial_, kRedBlocks, dev_out);
+        k_reduce_final<<<1, RED_FINAL_THREADS, 0, s>>>(partial_, kRedBlocks, dev_out);
     }
     void reset_counters(cudaStream_t s) override {
         cudaMemsetAsync(counters_, 0, sizeof(unsigned long long) * 2, s);

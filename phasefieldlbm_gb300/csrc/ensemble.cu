@@ -699,7 +699,7 @@ int pflbm_ensemble_reduce(pflbm_ensemble *e, int32_t box, pflbm_diag *d) {
     e->enqueue_analysis_box(box);
     pflbm::k_reduce_partial<float><<<Ensemble::kRedBlocks, pflbm::RED_THREADS, 0, e->stream>>>(e->boxes[box].p, e->macro,
                                                                                                e->partial);
-    pflbm::k_reduce_final<<<1, 32, 0, e->stream>>>(e->partial, Ensemble::kRedBlocks, e->dev_diag);
+    pflbm::k_reduce_final<<<1, pflbm::RED_FINAL_THREADS, 0, e->stream>>>(e->partial, Ensemble::kRedBlocks, e->dev_diag);
     double r[12];
     cudaMemcpyAsync(r, e->dev_diag, sizeof r, cudaMemcpyDeviceToHost, e->stream);
     const cudaError_t ce = cudaStreamSynchronize(e->stream);

@@ -162,42 +162,34 @@ constexpr int RED_THREADS = 256;
 
 template <class T>
 __global__ void __launch_bounds__(RED_THREADS) k_reduce_partial(const Params<T> p, const T *macro, double *partial) {
-    const int nx = p.nx, ny = p.ny, nz = p.nz;
-    const uint64_t N = p.Nd;
-    const uint64_t nint = static_cast<uint64_t>(nx - 2) * (ny - 2) * (nz - 2);
-    double acc[RED_FIELDS] = {0};
-    for (uint64_t k = blockIdx.x * static_cast<uint64_t>(RED_THREADS) + threadIdx.x; k < nint;
-         k += static_cast<uint64_t>(gridDim.x) * RED_THREADS) {
-        const uint64_t xi = k % (nx - 2), r = k / (nx - 2);
-        const uint64_t yi = r % (ny - 2), zi = r / (ny - 2);
-        const uint64_t i = (xi + 1) + static_cast<uint64_t>(nx) * ((yi + 1) + static_cast<uint64_t>(ny) * (zi + 1));
-        const double phi = macro[M_PHI * N + i], rho = macro[M_RHO * N + i];
-        const double ux = macro[M_UX * N + i], uy = macro[M_UY * N + i], uz = macro[M_UZ * N + i];
-        if (!isfinite(phi) || !isfinite(rho) || !isfinite(ux) || !isfinite(uy) || !isfinite(uz)) {
-            acc[10] += 1.0;
-            continue;
-        }
-        acc[0] += phi;
-        acc[1] += rho;
-        acc[2] += rho * ux;
-        acc[3] += rho * uy;
-        acc[4] += rho * uz;
-        acc[5] = fmax(acc[5], sqrt(ux * ux + uy * uy + uz * uz));
-        if (phi > 0.9) { acc[6] += rho; acc[7] += 1.0; }
-        if (phi < 0.1) { acc[8] += rho; acc[9] += 1.0; }
+    const uint32_t wx = p.nx - 2, wy = p.ny - 2;
+    const uint64_t N = p.Nd, nint = uint64_t(wx) * wy * (p.nz - 2);
+    const uint64_t first = blockIdx.x * uint64_t(RED_THREADS) + threadIdx.x, stride = uint64_t(gridDim.x) * RED_THREADS;
+    RedAcc acc;
+    // node k and the stride as (x, y, z) of the interior, carried on by
+    // additions: no division per node
+    uint32_t x = uint32_t(first % wx), y = uint32_t(first / wx % wy), z = uint32_t(first / wx / wy);
+    const uint32_t sx = uint32_t(stride % wx), sy = uint32_t(stride / wx % wy), sz = uint32_t(stride / wx / wy);
+    for (uint64_t k = first; k < nint; k += stride) {
+        const uint64_t i = (x + 1) + uint64_t(p.nx) * ((y + 1) + uint64_t(p.ny) * (z + 1));
+        acc.add(macro[M_RHO * N + i], macro[M_UX * N + i], macro[M_UY * N + i], macro[M_UZ * N + i],
+                macro[M_PHI * N + i]);
+        x += sx;
+        y += sy;
+        z += sz;
+        if (x >= wx) x -= wx, ++y;
+        if (y >= wy) y -= wy, ++z;
     }
-    block_reduce_row<RED_THREADS>(acc, partial + size_t(blockIdx.x) * RED_FIELDS);
+    double row[RED_FIELDS];
+    acc.row(row);
+    block_reduce_row<RED_THREADS>(row, partial + size_t(blockIdx.x) * RED_FIELDS);
 }
 
-static __global__ void __launch_bounds__(32) k_reduce_final(const double *partial, int nblocks, double *out) {
-    const int f = threadIdx.x;
-    if (f >= RED_FIELDS) return;
-    double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) {
-        const double v = partial[b * RED_FIELDS + f];
-        s = red_combine(f, s, v);
-    }
-    out[f] = s;
+static __global__ void __launch_bounds__(RED_FINAL_THREADS) k_reduce_final(const double *partial, int nblocks,
+                                                                           double *out) {
+    const int f = threadIdx.x >> 5;
+    const double s = red_total(partial, nblocks, f);
+    if ((threadIdx.x & 31) == 0) out[f] = s;
 }
 
 }  // namespace pflbm

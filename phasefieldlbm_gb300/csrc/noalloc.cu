@@ -130,42 +130,26 @@ __global__ void __launch_bounds__(kThreads)
     const int z = 1 + blockIdx.x;
     const int wx = nx - 2;
     const int n_plane = wx * (ny - 2);
-    double acc[kFields] = {0};
+    pflbm::RedAcc acc;
     for (int k = threadIdx.x; k < n_plane; k += kThreads) {
         const int x = 1 + k % wx, y = 1 + k / wx;
         const size_t i = size_t(x) + size_t(nx) * (size_t(y) + size_t(ny) * size_t(z));
-        const double f = phi[i], r = rho[i], vx = ux[i], vy = uy[i], vz = uz[i];
-        if (!isfinite(f) || !isfinite(r) || !isfinite(vx) || !isfinite(vy) || !isfinite(vz)) {
-            acc[10] += 1.0;
-            continue;
-        }
-        acc[0] += f;
-        acc[1] += r;
-        acc[2] += r * vx;
-        acc[3] += r * vy;
-        acc[4] += r * vz;
-        acc[5] = fmax(acc[5], sqrt(vx * vx + vy * vy + vz * vz));
-        if (f > 0.9) { acc[6] += r; acc[7] += 1.0; }
-        if (f < 0.1) { acc[8] += r; acc[9] += 1.0; }
+        acc.add(rho[i], ux[i], uy[i], uz[i], phi[i]);
     }
-    pflbm::block_reduce_row<kThreads>(acc, rows + size_t(blockIdx.x) * kFields);
+    double row[kFields];
+    acc.row(row);
+    pflbm::block_reduce_row<kThreads>(row, rows + size_t(blockIdx.x) * kFields);
 }
 
-// Sums the rows in plane order and writes the pflbm_diag the host entry point
+// Sums the rows and writes the pflbm_diag the host entry point
 // pflbm_reduce would produce (step = 0: fields carry no step count).
-__global__ void __launch_bounds__(32) k_reduce_rows(const double *__restrict__ rows, int n_rows, pflbm_diag *out) {
+__global__ void __launch_bounds__(pflbm::RED_FINAL_THREADS) k_reduce_rows(const double *__restrict__ rows, int n_rows,
+                                                                          pflbm_diag *out) {
     __shared__ double tot[kFields];
-    const int f = threadIdx.x;
-    if (f < kFields) {
-        double s = 0.0;
-        for (int b = 0; b < n_rows; ++b) {
-            const double v = rows[size_t(b) * kFields + f];
-            s = pflbm::red_combine(f, s, v);
-        }
-        tot[f] = s;
-    }
+    const double s = pflbm::red_total(rows, n_rows, threadIdx.x >> 5);
+    if ((threadIdx.x & 31) == 0) tot[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (f == 0) {
+    if (threadIdx.x == 0) {
         pflbm_diag d;
         d.step = 0;
         d.phi_mass = tot[0];
@@ -209,7 +193,7 @@ extern "C" int pflbm_reduce_fields_noalloc(const float *rho, const float *ux, co
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int planes = nz - 2;
     k_reduce_planes<<<planes, kThreads, 0, s>>>(rho, ux, uy, uz, phi, nx, ny, rows);
-    k_reduce_rows<<<1, 32, 0, s>>>(rows, planes, dev_out);
+    k_reduce_rows<<<1, pflbm::RED_FINAL_THREADS, 0, s>>>(rows, planes, dev_out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "pflbm_reduce_fields_noalloc launch");
     return PFLBM_OK;
