@@ -77,6 +77,8 @@ struct pflbm_sim {
     uint64_t step = 0;       // completed steps
     bool initialized = false;
     int64_t cache_step = -1; // step the analysis cache describes
+    bool cache_full = false; // all 18 arrays of it, or rho, u, phi and |grad phi|
+    bool wants_full = false; // some field beyond those has been read: rebuild all 18 at once
     bool distros_dirty = false; // initial fields changed since the last rebuild
     double *dev_diag = nullptr;
     // background output writer (pflbm_write_output_async)
@@ -238,18 +240,22 @@ void flush_initial(pflbm_sim *s) {
     }
 }
 
-int ensure_cache(pflbm_sim *s) {
-    if (s->cache_step == int64_t(s->step)) return PFLBM_OK;
-    if (s->step == 0 && s->cache_step == 0) {
-        // the cache still holds the initial fields
-        s->cache_step = 0;
-        return PFLBM_OK;
-    }
-    s->eng->enqueue_analysis(s->parity ^ 1, uint32_t(s->step - 1), s->stream);
+// Fields 0..17 that every analysis rebuilds (MODE_ANALYSIS_BASE).
+bool base_field(int32_t id) {
+    return id == PFLBM_FIELD_RHO || id == PFLBM_FIELD_UX || id == PFLBM_FIELD_UY || id == PFLBM_FIELD_UZ ||
+           id == PFLBM_FIELD_PHI || id == PFLBM_FIELD_IND;
+}
+
+int ensure_cache(pflbm_sim *s, bool full = false) {
+    if (full) s->wants_full = true;
+    // at step 0 the cache still holds the initial fields
+    if (s->cache_step == int64_t(s->step) && (s->cache_full || !full)) return PFLBM_OK;
+    s->eng->enqueue_analysis(s->parity ^ 1, uint32_t(s->step - 1), s->wants_full, s->stream);
     s->eng->enqueue_vorticity(s->stream);
     cudaError_t e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return cuda_fail(e, "analysis");
     s->cache_step = int64_t(s->step);
+    s->cache_full = s->wants_full;
     return PFLBM_OK;
 }
 
@@ -289,7 +295,7 @@ int get_field_impl(pflbm_sim *s, int32_t id, void *host, size_t bytes, bool as_d
     if (bytes < need) return fail(PFLBM_ERR_INVALID_ARG, "destination buffer too small");
     if (id < 0 || id >= PFLBM_FIELD_COUNT) return fail(PFLBM_ERR_INVALID_ARG, "unknown field id");
     const int rb = s->eng->real_bytes();
-    int rc = ensure_cache(s);
+    int rc = ensure_cache(s, id <= PFLBM_FIELD_FFZ && !base_field(id));
     if (rc) return rc;
     const unsigned char *src = nullptr;
     if (id <= PFLBM_FIELD_FFZ) {
@@ -552,6 +558,7 @@ int pflbm_init(pflbm_sim *s) {
     s->parity = 0;
     s->step = 0;
     s->cache_step = 0;
+    s->cache_full = true;
     s->distros_dirty = false;
     s->initialized = true;
     return PFLBM_OK;

@@ -45,8 +45,9 @@ class Engine {
     // Initial macroscopic fields into the cache, then f/phi from them.
     virtual void enqueue_init_fields(cudaStream_t s) = 0;
     virtual void enqueue_init_distros(cudaStream_t s) = 0;
-    // Rebuilds the reference's arrays after step t from ping-pong `parity`.
-    virtual void enqueue_analysis(int parity, uint32_t t, cudaStream_t s) = 0;
+    // Rebuilds the reference's arrays after step t from ping-pong `parity`:
+    // all 18 (`full`), or rho, u, phi and |grad phi|.
+    virtual void enqueue_analysis(int parity, uint32_t t, bool full, cudaStream_t s) = 0;
     virtual void enqueue_vorticity(cudaStream_t s) = 0;
     // FP64 diagnostics of the cache into out[12] (device pointer).
     virtual void enqueue_reduce(cudaStream_t s, double *dev_out) = 0;

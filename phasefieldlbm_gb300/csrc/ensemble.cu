@@ -502,10 +502,18 @@ class Ensemble {
                                                                       bp.phi[0] + bx.n_off, bp.phi[1] + bx.n_off, macro);
     }
 
-    // Analysis of one box after the last completed step into the macro cache.
-    void enqueue_analysis_box(int k) {
+    // Analysis of one box after the last completed step into the macro cache:
+    // all 18 arrays (`full`) or those of MODE_ANALYSIS_BASE. The cache holds
+    // one box at a time; a field of the box that it holds is read from it.
+    int cache_box = -1;
+    uint64_t cache_step = 0;
+    bool cache_full = false;
+    void enqueue_analysis_box(int k, bool full) {
+        if (cache_box == k && cache_step == step && (cache_full || !full)) return;
+        cache_box = k;
+        cache_step = step;
+        cache_full = full || step == 0;
         const Params<float> &p = boxes[k].p;
-        const dim3 blk(32, 8, 1), grd((p.nx + 31) / 32, (p.ny + 7) / 8, p.nz);
         if (step == 0) {
             enqueue_init_box(k);  // the cache then holds the initial fields
             return;
@@ -517,11 +525,17 @@ class Ensemble {
         b.t_fixed = uint32_t(step - 1);
         const int chunks = (int(p.nz) - 2 + p.zchunk - 1) / p.zchunk;
         const dim3 cg((p.nx + TX - 1) / TX, (p.ny + TY - 1) / TY, chunks);
-        if (q == 19)
-            k_collide<19, false, float, MODE_ANALYSIS><<<cg, dim3(TX, TY), 0, stream>>>(p, b);
+        const dim3 blk3(TX, TY);
+        if (full && q == 19)
+            k_collide<19, false, float, MODE_ANALYSIS><<<cg, blk3, 0, stream>>>(p, b);
+        else if (full)
+            k_collide<27, false, float, MODE_ANALYSIS><<<cg, blk3, 0, stream>>>(p, b);
+        else if (q == 19)
+            k_collide<19, false, float, MODE_ANALYSIS_BASE><<<cg, blk3, 0, stream>>>(p, b);
         else
-            k_collide<27, false, float, MODE_ANALYSIS><<<cg, dim3(TX, TY), 0, stream>>>(p, b);
-        k_analysis_ghosts<float><<<grd, blk, 0, stream>>>(p, 0, uint32_t(step - 1), macro);
+            k_collide<27, false, float, MODE_ANALYSIS_BASE><<<cg, blk3, 0, stream>>>(p, b);
+        const unsigned int shell = unsigned((shell_nodes(p.nx, p.ny, p.nz) + 255) / 256);
+        k_analysis_ghosts<float><<<shell, 256, 0, stream>>>(p, 0, uint32_t(step - 1), macro, full);
     }
 };
 
@@ -626,6 +640,7 @@ int pflbm_ensemble_init(pflbm_ensemble *e) {
     cudaMemsetAsync(e->bp.err, 0, sizeof(unsigned int) * 4, e->stream);
     cudaMemsetAsync(e->bp.gbar, 0, sizeof(pflbm::GridBar), e->stream);
     for (size_t k = 0; k < e->boxes.size(); ++k) e->enqueue_init_box(int(k));
+    e->cache_box = -1;
     const cudaError_t ce = cudaStreamSynchronize(e->stream);
     if (ce != cudaSuccess) return ecuda(ce, "ensemble init");
     e->parity = 0;
@@ -683,7 +698,9 @@ int pflbm_ensemble_get_field(pflbm_ensemble *e, int32_t box, int32_t id, void *h
     const uint64_t N = e->hps[box].N;
     if (bytes < N * sizeof(float)) return efail(PFLBM_ERR_INVALID_ARG, "destination buffer too small");
     cudaSetDevice(e->device);
-    e->enqueue_analysis_box(box);
+    const bool base = id == PFLBM_FIELD_RHO || id == PFLBM_FIELD_UX || id == PFLBM_FIELD_UY || id == PFLBM_FIELD_UZ ||
+                      id == PFLBM_FIELD_PHI || id == PFLBM_FIELD_IND;
+    e->enqueue_analysis_box(box, !base);
     const cudaError_t ce =
         cudaMemcpyAsync(host, e->macro + size_t(id) * N, N * sizeof(float), cudaMemcpyDeviceToHost, e->stream);
     if (ce != cudaSuccess) return ecuda(ce, "ensemble readback");
@@ -696,7 +713,7 @@ int pflbm_ensemble_reduce(pflbm_ensemble *e, int32_t box, pflbm_diag *d) {
     if (!e || !d) return efail(PFLBM_ERR_INVALID_ARG, "null argument");
     if (box < 0 || box >= int32_t(e->boxes.size())) return efail(PFLBM_ERR_INVALID_ARG, "box index out of range");
     cudaSetDevice(e->device);
-    e->enqueue_analysis_box(box);
+    e->enqueue_analysis_box(box, false);
     pflbm::k_reduce_partial<float><<<Ensemble::kRedBlocks, pflbm::RED_THREADS, 0, e->stream>>>(e->boxes[box].p, e->macro,
                                                                                                e->partial);
     pflbm::k_reduce_final<<<1, pflbm::RED_FINAL_THREADS, 0, e->stream>>>(e->partial, Ensemble::kRedBlocks, e->dev_diag);

@@ -57,7 +57,12 @@ constexpr int TX = PFLBM_TILE_X, TY = PFLBM_TILE_Y, NT = TX * TY;
 constexpr int PX = TX + 4, PY = TY + 4;  // phi tile + halo 2
 constexpr int NX_ = TX + 2, NY_ = TY + 2;  // normal tile + halo 1
 
-enum Mode { MODE_STEP = 0, MODE_STEP_AVG = 1, MODE_ANALYSIS = 2, MODE_STEP_CLOSURE = 3, MODE_STEP_CLOSURE_AVG = 4 };
+// The readback modes write the reference's arrays instead of advancing:
+// MODE_ANALYSIS all 18, MODE_ANALYSIS_BASE rho, u, phi and |grad phi|, which
+// is what outputs, diagnostics, vorticity and training snapshots read.
+enum Mode { MODE_STEP = 0, MODE_STEP_AVG = 1, MODE_ANALYSIS = 2, MODE_STEP_CLOSURE = 3, MODE_STEP_CLOSURE_AVG = 4,
+            MODE_ANALYSIS_BASE = 5 };
+constexpr bool mode_analysis(int m) { return m == MODE_ANALYSIS || m == MODE_ANALYSIS_BASE; }
 constexpr bool mode_closure(int m) { return m == MODE_STEP_CLOSURE || m == MODE_STEP_CLOSURE_AVG; }
 constexpr bool mode_average(int m) { return m == MODE_STEP_AVG || m == MODE_STEP_CLOSURE_AVG; }
 
@@ -96,7 +101,7 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
     const T fx = st * n_x, fy = st * n_y, fz = st * n_z;
 
     // moments (src/lbm.cu:33-128)
-    const Macro<T> m = moments<QQ, T>(pop, fx, fy, fz);
+    const Macro<T> m = moments<QQ, T, mode_analysis(MODE)>(pop, fx, fy, fz);
 
     // learned eddy viscosity nu_cl = strength * nu_t, as a relaxation-time
     // increment tau_t = 3 nu_cl (tau = 1/2 + 3 nu)
@@ -127,7 +132,16 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
     }
     const CollideCtx<T> k = make_ctx<QQ, T>(m, fx, fy, fz, T(1) - omega);
 
-    if constexpr (MODE == MODE_ANALYSIS) {
+    if constexpr (MODE == MODE_ANALYSIS_BASE) {
+        T *mc = b.macro;
+        mc[M_RHO * Nd + dense] = m.rho;
+        mc[M_UX * Nd + dense] = m.ux;
+        mc[M_UY * Nd + dense] = m.uy;
+        mc[M_UZ * Nd + dense] = m.uz;
+        mc[M_PHI * Nd + dense] = phi;
+        mc[M_IND * Nd + dense] = ind;
+        return;
+    } else if constexpr (MODE == MODE_ANALYSIS) {
         T *mc = b.macro;
         mc[M_RHO * Nd + dense] = m.rho;
         mc[M_UX * Nd + dense] = m.ux;

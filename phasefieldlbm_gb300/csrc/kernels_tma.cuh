@@ -253,7 +253,10 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
     // of that warp computes normal-ring entries, so that with the 3-plane
     // ring the copies are issued while the other warps compute the normals
     // between the plane's two barriers, not by a warp on that critical path.
-    constexpr int kNormWork = sizeof(T) == 4 ? NXP * NY_ : NX_ * NY_;
+    // packed normals (two entries per thread); the readback modes evaluate them
+    // one by one, as the plain-load kernel does, down to the last denormal
+    constexpr bool kPacked = sizeof(T) == 4 && !mode_analysis(MODE);
+    constexpr int kNormWork = kPacked ? NXP * NY_ : NX_ * NY_;
     constexpr int kIssuer = kNormWork <= NT - 32 ? NT - 32 : 0;
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::off_bar);
     volatile int *s_abort = reinterpret_cast<volatile int *>(smem + L::off_bar + 8 * NS);
@@ -309,7 +312,7 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
     auto compute_n = [&](int zp) {
         const int sn = pslot(zp), sm = pslot(zp - 1), sp = pslot(zp + 1);
         const int nn = nslot(zp);
-        if constexpr (sizeof(T) == 4) {
+        if constexpr (kPacked) {
             // two x-adjacent entries per thread: 170 entry pairs, at most one
             // per thread, so no warp computes a second round
             const bool zok = zp >= 1 && zp <= nz - 2;
@@ -337,8 +340,8 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
                     auto v = [&](int dx, int dy, int dz) -> T {
                         return phi_at(dz < 0 ? sm : (dz > 0 ? sp : sn), ly + 1 + dy, lx + L::PXO - 1 + dx);
                     };
-                    unit_normal<false>(lattice_grad<QQ, 0, T>(v), lattice_grad<QQ, 1, T>(v), lattice_grad<QQ, 2, T>(v),
-                                       nxv, nyv, nzv, ind);
+                    unit_normal<sizeof(T) == 4>(lattice_grad<QQ, 0, T>(v), lattice_grad<QQ, 1, T>(v),
+                                                lattice_grad<QQ, 2, T>(v), nxv, nyv, nzv, ind);
                 }
                 n_at(0, nn, ly, lx) = nxv;
                 n_at(1, nn, ly, lx) = nyv;

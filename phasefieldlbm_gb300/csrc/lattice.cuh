@@ -23,6 +23,19 @@
 
 namespace pflbm {
 
+// Correctly rounded elementary operations (never contracted), so that the
+// scalar stencils and their packed two-lane form (V2, packed.cuh) round
+// identically and the kernels built on either agree bit for bit. The
+// compiler fuses a packed multiply followed by a packed add into one FFMA2
+// even when both carry .rn, so the stencils below never feed a product into
+// an addition: every multiply-add is written as op_fma.
+__device__ __forceinline__ float op_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double op_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float op_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double op_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float op_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double op_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+
 // ---- direction table (27 entries; D3Q19 uses the first 19) ---------------
 __device__ constexpr int kCX[27] = {0, 1, -1, 0, 0, 0, 0, 1, -1, 1, -1, 0, 0, 1, -1, 1, -1, 0, 0, 1, -1, 1, -1, 1, -1, -1, 1};
 __device__ constexpr int kCY[27] = {0, 0, 0, 1, -1, 0, 0, 1, -1, 0, 0, 1, -1, -1, 1, 0, 0, 1, -1, 1, -1, 1, -1, -1, 1, 1, -1};
@@ -57,7 +70,10 @@ struct Macro {
 // through the sums s_k = f_(2k-1) + f_(2k) and differences d_k = f_(2k-1) -
 // f_(2k) of the opposite pairs: first moments are sums of d_k, second
 // moments sums of s_k (c_a c_b is the same for q and its opposite).
-template <int QQ, class T>
+// ROUNDED fixes the rounding of u (no contraction left to the compiler), so
+// that the readback kernels agree to the last denormal however they are fed
+// and however many of the arrays they write.
+template <int QQ, class T, bool ROUNDED = false>
 __device__ __forceinline__ Macro<T> moments(const T (&f)[QQ], T fx, T fy, T fz) {
     constexpr int NP = (QQ - 1) / 2;
     T sp[NP], dp[NP];
@@ -93,10 +109,20 @@ __device__ __forceinline__ Macro<T> moments(const T (&f)[QQ], T fx, T fy, T fz) 
         if (cy * cz < 0) myz -= sp[k];
     }
     const T inv = T(1) / rho;
-    T ux = inv * jx, uy = inv * jy, uz = inv * jz;
-    ux += fx * T(0.5) * inv;
-    uy += fy * T(0.5) * inv;
-    uz += fz * T(0.5) * inv;
+    T ux, uy, uz;
+    if constexpr (ROUNDED) {
+        // (halving inv, not the force: a halved product may be rounded once or
+        // twice where it is denormal)
+        const T half = op_mul(inv, T(0.5));
+        ux = op_fma(fx, half, op_mul(inv, jx));
+        uy = op_fma(fy, half, op_mul(inv, jy));
+        uz = op_fma(fz, half, op_mul(inv, jz));
+    } else {
+        ux = inv * jx, uy = inv * jy, uz = inv * jz;
+        ux += fx * T(0.5) * inv;
+        uy += fy * T(0.5) * inv;
+        uz += fz * T(0.5) * inv;
+    }
     T pxx = mxx - rho * ux * ux + ux * fx;
     T pyy = myy - rho * uy * uy + uy * fy;
     T pzz = mzz - rho * uz * uz + uz * fz;

@@ -9,18 +9,6 @@
 
 namespace pflbm {
 
-// Correctly rounded elementary operations (never contracted), so that the
-// scalar stencils and their packed two-lane form (V2, packed.cuh) round
-// identically and the kernels built on either agree bit for bit. The
-// compiler fuses a packed multiply followed by a packed add into one FFMA2
-// even when both carry .rn, so the stencils below never feed a product into
-// an addition: every multiply-add is written as op_fma.
-__device__ __forceinline__ float op_mul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double op_mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float op_add(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double op_add(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float op_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double op_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float op_sqrt(float a) { return sqrtf(a); }
 // approximate square root (PTX sqrt.approx.f32, about 2 ulp): the FAST
 // normals of FP32-arithmetic runs
