@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(G::NT, batch_min_blocks<G>())
     const int tid = threadIdx.x + G::TX * threadIdx.y;
     if (blockIdx.x == 0 && tid == 0) bp.ctr[1] = 0u;
     tma_pipeline_init<QQ, float, L>(smem);
-    uint32_t seq = 0;
+    uint32_t seq = 0, tiles = 0;
     for (;;) {
         if (tid == 0) *s_item = int(atomicAdd(&bp.ctr[0], 1u));
         __syncthreads();
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(G::NT, batch_min_blocks<G>())
         const BoxDev &bx = boxes[w.box];
         const StepBuffers<float, float> b = box_buffers(bp, bx, parity);
         if (!collide_tile_tma<QQ, false, float, MODE_STEP, G, L>(bx.p, b, &maps.fn[w.box], &maps.fw[w.box],
-                                                             &maps.phi[w.box], w.x0, w.y0, w.zb, w.ze, smem, seq))
+                                                             &maps.phi[w.box], w.x0, w.y0, w.zb, w.ze, smem, seq, tiles))
             return;
         __syncthreads();  // shared rings are reused by the next item
     }

@@ -525,18 +525,14 @@ __device__ __forceinline__ bool collide_tile_pair(const Params<float> &p, const 
         tma_prefetch_desc(fmapw_p);
         tma_prefetch_desc(phimap_p);
     }
-    for (int zp = zb - 2; zp <= zb + 1; ++zp) {
-        const int slot = pslot(zp);
-        for (int i = tid; i < L::PBW * L::PBH; i += NT2) {
-            const int lx = i % L::PBW, ly = i / L::PBW;
-            const int gx = x0 - L::PXO + lx, gy = y0 - 2 + ly;
-            T v = T(0);
-            if (gx >= 0 && gx < nx && gy >= 0 && gy < ny && zp >= 0 && zp < nz)
-                v = b.phi_src[gx + static_cast<uint64_t>(nx) * (gy + static_cast<uint64_t>(ny) * zp)];
-            phi_at(slot, ly, lx) = v;
-        }
+    // first phi planes and stages by TMA, as collide_tile_tma
+    if (tid == kIssuer) {
+        fence_proxy_async();
+        mbar_arrive_expect_tx(warm_bar<L>(smem), uint32_t(4 * L::phi_plane_bytes));
+        for (int zp = zb - 2; zp <= zb + 1; ++zp)
+            tma_load_3d(&phi_at(pslot(zp), 0, 0), phimap_p, warm_bar<L>(smem), x0 - L::PXO, y0 - 2, zp);
+        for (int k = 0; k < NS - 2 && zb + k < ze; ++k) issue((seq + k) % NS, zb + k);
     }
-    fence_proxy_async();
     // normals of plane zp on the tile + halo 1, two x-adjacent entries per
     // thread (entry pairs start at even lx, so the +-1 neighbours of the pair
     // are aligned 8-byte words and only the dx = 0 column needs two loads)
@@ -562,11 +558,19 @@ __device__ __forceinline__ bool collide_tile_pair(const Params<float> &p, const 
             if (ly >= 1 && ly <= TY) *reinterpret_cast<float2 *>(&ind_at(zp, ly - 1, lx)) = indv.v;
         }
     };
-    __syncthreads();
+    if (!plane_wait<L>(smem, warm_bar<L>(smem), 0)) *s_abort = 1;
     compute_n(zb - 1);
     __syncthreads();
-    if (tid == kIssuer)
-        for (int k = 0; k < NS - 1 && zb + k < ze; ++k) issue((seq + k) % NS, zb + k);
+    if (*s_abort) {
+        if (tid == 0) {
+            atomicOr(b.err, 1u);
+            mbar_wait_bounded(warm_bar<L>(smem), 0, kWaitLimit);
+            for (int k = 0; k < NS - 2 && zb + k < ze; ++k)
+                mbar_wait_bounded(&bar[(seq + k) % NS], ((seq + k) / NS) & 1, kWaitLimit);
+        }
+        return false;
+    }
+    if (tid == kIssuer && zb + NS - 2 < ze) issue((seq + NS - 2) % NS, zb + NS - 2);
     compute_n(zb);
 
     for (int z = zb; z < ze; ++z) {

@@ -130,8 +130,9 @@ struct TmaPlan {
     static constexpr size_t off_ind = align128(off_n + n_bytes);
     static constexpr size_t ind_bytes = size_t(3) * TY * NX_ * sizeof(RT);
     static constexpr size_t off_bar = align128(off_ind + ind_bytes);
-    // NS mbarriers, the abort flag, and at off_bar + 64 the test build's
-    // never-arriving barrier (plane_wait)
+    // NS mbarriers, the abort flag, at off_bar + 64 the test build's
+    // never-arriving barrier (plane_wait), at off_bar + 96 the barrier of a
+    // tile's first phi planes
     static constexpr size_t total = off_bar + 128;
     static constexpr uint32_t tx_bytes = uint32_t(f_bytes() + phi_plane_bytes);
     static_assert(stage_bytes % 128 == 0 && phi_slot_bytes % 128 == 0 && off_phi % 128 == 0, "TMA smem alignment");
@@ -198,12 +199,19 @@ template <int QQ, class S, int MODE>
 using TmaModeLayout = typename std::conditional<mode_closure(MODE), TmaPlan<QQ, S, TmaClosureStages<QQ, S>::value>,
                                                 TmaLayout<QQ, S>>::type;
 
+// The barrier of a tile's first phi planes.
+template <class L>
+__device__ __forceinline__ uint64_t *warm_bar(unsigned char *smem) {
+    return reinterpret_cast<uint64_t *>(smem + L::off_bar + 96);
+}
+
 // Barriers of the TMA pipeline: once per CTA, before its first tile.
 template <int QQ, class S, class L = TmaLayout<QQ, S>>
 __device__ __forceinline__ void tma_pipeline_init(unsigned char *smem) {
     if (threadIdx.x + blockDim.x * threadIdx.y == 0) {
         uint64_t *bar = reinterpret_cast<uint64_t *>(smem + L::off_bar);
         for (int k = 0; k < L::kStages; ++k) mbar_init(&bar[k], 1);
+        mbar_init(warm_bar<L>(smem), 1);
         *reinterpret_cast<volatile int *>(smem + L::off_bar + 8 * L::kStages) = 0;
 #ifdef PFLBM_TEST_DEAD_WAIT
         mbar_init(reinterpret_cast<uint64_t *>(smem + L::off_bar + 64), 1);
@@ -233,14 +241,16 @@ __device__ __forceinline__ bool plane_wait(unsigned char *smem, uint64_t *bar, u
 // One column tile [x0, x0+TX) x [y0, y0+TY), planes zb .. ze-1. `seq` counts
 // the stages this CTA has consumed so far (stage = seq % NS, mbarrier phase
 // parity = (seq / NS) & 1), so that a persistent CTA can run tile after tile
-// on the same barriers; every stage issued for a tile is consumed by it.
+// on the same barriers; every stage issued for a tile is consumed by it, and
+// `tiles` counts the tiles begun.
 // Returns false when a bounded wait gave up (error word set, copies drained).
 template <int QQ, bool JET, class S, int MODE, class G = DefaultTile, class L = TmaLayout<QQ, S, G>>
 __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>::T> &p,
                                                  const StepBuffers<S, typename Store<S>::T> &b,
                                                  const CUtensorMap *fmapn_p, const CUtensorMap *fmapw_p,
                                                  const CUtensorMap *phimap_p, int x0, int y0, int zb, int ze,
-                                                 unsigned char *smem, uint32_t &seq, float *s_mlp = nullptr) {
+                                                 unsigned char *smem, uint32_t &seq, uint32_t &tiles,
+                                                 float *s_mlp = nullptr) {
     using T = typename Store<S>::T;
     static_assert(std::is_same<typename L::Tile, G>::value, "plan for this tile");
     constexpr int TX = G::TX, TY = G::TY, NT = G::NT, NX_ = G::NX, NY_ = G::NY, NXP = G::NXP;
@@ -295,20 +305,21 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
         tma_prefetch_desc(phimap_p);
     }
 
-    // warm-up: phi planes zb-2 .. zb+1 with plain loads, normals of zb-1, zb
-    for (int zp = zb - 2; zp <= zb + 1; ++zp) {
-        const int slot = pslot(zp);
-        for (int i = tid; i < L::PBW * L::PBH; i += NT) {
-            const int lx = i % L::PBW, ly = i / L::PBW;
-            const int gx = x0 - L::PXO + lx, gy = y0 - 2 + ly;
-            T v = T(0);
-            if (gx >= 0 && gx < nx && gy >= 0 && gy < ny && zp >= 0 && zp < nz)
-                v = b.phi_src[gx + static_cast<uint64_t>(p.px) * (gy + static_cast<uint64_t>(ny) * zp)];
-            phi_at(slot, ly, lx) = v;
-        }
+    // warm-up: phi planes zb-2 .. zb+1, then the normals of zb-1 and zb. The
+    // four planes come by TMA in one go, and with them the first NS-2 stages
+    // (their phi planes fill the rest of the ring), so that the tile waits
+    // once for memory before it starts. Loaded element by element by all
+    // threads, and the stages after the first normals, the warm-up took as
+    // long as three planes (64x64x128 D3Q19 jet, one wave of 7-plane chunks:
+    // collide 20.7 -> 18.8 us; 128^3 droplet 74.8 -> 68.7; D3Q27 128x128x512
+    // 372 -> 358).
+    if (tid == kIssuer) {
+        fence_proxy_async();
+        mbar_arrive_expect_tx(warm_bar<L>(smem), uint32_t(4 * L::phi_plane_bytes));
+        for (int zp = zb - 2; zp <= zb + 1; ++zp)
+            tma_load_3d(&phi_at(pslot(zp), 0, 0), phimap_p, warm_bar<L>(smem), x0 - L::PXO, y0 - 2, zp);
+        for (int k = 0; k < NS - 2 && zb + k < ze; ++k) issue((seq + k) % NS, zb + k);
     }
-    // these generic writes precede later TMA writes to the same ring slots
-    fence_proxy_async();
     auto compute_n = [&](int zp) {
         const int sn = pslot(zp), sm = pslot(zp - 1), sp = pslot(zp + 1);
         const int nn = nslot(zp);
@@ -350,13 +361,22 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
             }
         }
     };
-    __syncthreads();
+    if (!plane_wait<L>(smem, warm_bar<L>(smem), tiles & 1)) *s_abort = 1;
     compute_n(zb - 1);
     __syncthreads();
-    // stages 0 .. NS-2 (planes zb .., phi zb+2 ..); the phi ring slot of
-    // plane zb+NS aliases that of zb-2, which compute_n(zb-1) no longer needs
-    if (tid == kIssuer)
-        for (int k = 0; k < NS - 1 && zb + k < ze; ++k) issue((seq + k) % NS, zb + k);
+    if (*s_abort) {
+        if (tid == 0) {
+            atomicOr(b.err, 1u);
+            mbar_wait_bounded(warm_bar<L>(smem), tiles & 1, kWaitLimit);
+            for (int k = 0; k < NS - 2 && zb + k < ze; ++k)
+                mbar_wait_bounded(&bar[(seq + k) % NS], ((seq + k) / NS) & 1, kWaitLimit);
+        }
+        return false;
+    }
+    ++tiles;
+    // stage NS-2: the phi ring slot of plane zb+NS aliases that of zb-2, which
+    // compute_n(zb-1) no longer needs
+    if (tid == kIssuer && zb + NS - 2 < ze) issue((seq + NS - 2) % NS, zb + NS - 2);
     compute_n(zb);
 
     for (int z = zb; z < ze; ++z) {
@@ -443,9 +463,9 @@ __global__ void __launch_bounds__(NT, CollideOccupancy<QQ, S>::value)
     tma_pipeline_init<QQ, S, L>(smem);
     const int zb = 1 + blockIdx.z * p.zchunk;
     const int ze = min(zb + p.zchunk, int(p.nz) - 1);
-    uint32_t seq = 0;
+    uint32_t seq = 0, tiles = 0;
     collide_tile_tma<QQ, JET, S, MODE, DefaultTile, L>(p, b, &fmapn, &fmapw, &phimap, int(blockIdx.x) * TX,
-                                                       int(blockIdx.y) * TY, zb, ze, smem, seq, s_mlp);
+                                                       int(blockIdx.y) * TY, zb, ze, smem, seq, tiles, s_mlp);
 }
 
 }  // namespace pflbm
