@@ -46,6 +46,7 @@
 #include "boundary.cuh"
 #include "closure_net.cuh"
 #include "lattice.cuh"
+#include "lattice_f64.cuh"
 #include "params.cuh"
 #include "sround.cuh"
 #include "stencil.cuh"
@@ -101,7 +102,11 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
     const T fx = st * n_x, fy = st * n_y, fz = st * n_z;
 
     // moments (src/lbm.cu:33-128)
-    const Macro<T> m = moments<QQ, T, mode_analysis(MODE)>(pop, fx, fy, fz);
+    Macro<T> m;
+    if constexpr (sizeof(T) == 8)
+        m = moments_f64<QQ>(pop, fx, fy, fz);
+    else
+        m = moments<QQ, T, mode_analysis(MODE)>(pop, fx, fy, fz);
 
     // learned eddy viscosity nu_cl = strength * nu_t, as a relaxation-time
     // increment tau_t = 3 nu_cl (tau = 1/2 + 3 nu)
@@ -122,16 +127,18 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
     T omega;
     if constexpr (JET) {
         const T tau_phi = (T(1) - phi) * p.tau_water + phi * p.tau_oil + tau_t;
-        const T r = sponge_ramp<T>(p, z);
-        const T visc_local = (T(1) - phi) * p.visc_water + phi * p.visc_oil;
-        const T tau_zmax = T(0.5) + T(3) * (visc_local * p.kgain1);
-        const T tau_eff = tau_phi + r * (tau_zmax - tau_phi);
-        omega = T(1) / tau_eff;
+        if (sizeof(T) == 8 && !(static_cast<T>(z) * p.inv_nz_m1 > p.z_start)) {
+            omega = T(1) / tau_phi;  // below the sponge (FP64 instructions saved; r = 0 gives the same)
+        } else {
+            const T r = sponge_ramp<T>(p, z);
+            const T visc_local = (T(1) - phi) * p.visc_water + phi * p.visc_oil;
+            const T tau_zmax = T(0.5) + T(3) * (visc_local * p.kgain1);
+            const T tau_eff = tau_phi + r * (tau_zmax - tau_phi);
+            omega = T(1) / tau_eff;
+        }
     } else {
         omega = tau_t == T(0) ? p.omega_ref : T(1) / (T(1) / p.omega_ref + tau_t);
     }
-    const CollideCtx<T> k = make_ctx<QQ, T>(m, fx, fy, fz, T(1) - omega);
-
     if constexpr (MODE == MODE_ANALYSIS_BASE) {
         T *mc = b.macro;
         mc[M_RHO * Nd + dense] = m.rho;
@@ -202,14 +209,22 @@ __device__ __forceinline__ void collide_node(const Params<typename Store<S>::T> 
                 Store<S>::store(b.f_dst + uint64_t(q) * N, idx, v, inv_w);
             }
         };
-        if (PFLBM_GUARD(base < N, b.err)) put(0, node, collide_rest<QQ, T>(k));
+        if constexpr (sizeof(T) == 8) {
+            collide_f64<QQ>(m, fx, fy, fz, T(1) - omega, [&](int q, T v) {
+                const uint32_t i = q == 0 ? node : dst_node(q);
+                if (PFLBM_GUARD(i < N, b.err)) put(q, i, v);
+            });
+        } else {
+            const CollideCtx<T> k = make_ctx<QQ, T>(m, fx, fy, fz, T(1) - omega);
+            if (PFLBM_GUARD(base < N, b.err)) put(0, node, collide_rest<QQ, T>(k));
 #pragma unroll
-        for (int q = 1; q < QQ; q += 2) {
-            T a, c;
-            collide_pair<QQ, T>(q, k, a, c);
-            const uint32_t iq = dst_node(q), iqb = dst_node(q + 1);
-            if (PFLBM_GUARD(iq < N, b.err)) put(q, iq, a);
-            if (PFLBM_GUARD(iqb < N, b.err)) put(q + 1, iqb, c);
+            for (int q = 1; q < QQ; q += 2) {
+                T a, c;
+                collide_pair<QQ, T>(q, k, a, c);
+                const uint32_t iq = dst_node(q), iqb = dst_node(q + 1);
+                if (PFLBM_GUARD(iq < N, b.err)) put(q, iq, a);
+                if (PFLBM_GUARD(iqb < N, b.err)) put(q + 1, iqb, c);
+            }
         }
         // phase flux (src/lbm.cu:209-238): g_q = w_q (phi + c_q . J). With the
         // closure's phase mixing, the sub-filter flux -D_t grad phi, D_t =
@@ -342,8 +357,14 @@ __device__ __forceinline__ void collide_tile(const Params<typename Store<S>::T> 
                 };
                 // FP32: approximate square root and reciprocal, as the TMA
                 // kernel's packed normals (bit-identical); FP64: IEEE
-                unit_normal<sizeof(T) == 4>(lattice_grad<QQ, 0, T>(v), lattice_grad<QQ, 1, T>(v), lattice_grad<QQ, 2, T>(v), nxv,
-                                   nyv, nzv, ind);
+                if constexpr (sizeof(T) == 8) {
+                    T gx, gy, gz;
+                    gradient_f64<QQ>(v, gx, gy, gz);
+                    unit_normal_f64(gx, gy, gz, nxv, nyv, nzv, ind);
+                } else {
+                    unit_normal<true>(lattice_grad<QQ, 0, T>(v), lattice_grad<QQ, 1, T>(v), lattice_grad<QQ, 2, T>(v),
+                                      nxv, nyv, nzv, ind);
+                }
             }
             s_n[0][sn][ly][lx] = nxv;
             s_n[1][sn][ly][lx] = nyv;
@@ -393,10 +414,15 @@ __device__ __forceinline__ void collide_tile(const Params<typename Store<S>::T> 
         auto nv = [&](int c, int dx, int dy, int dz) -> T {
             return s_n[c][dz < 0 ? s_m : (dz > 0 ? s_p : s_0)][ty + 1 + dy][tx + 1 + dx];
         };
-        const T scx = lattice_grad<QQ, 0, T>([&](int dx, int dy, int dz) { return nv(0, dx, dy, dz); });
-        const T scy = lattice_grad<QQ, 1, T>([&](int dx, int dy, int dz) { return nv(1, dx, dy, dz); });
-        const T scz = lattice_grad<QQ, 2, T>([&](int dx, int dy, int dz) { return nv(2, dx, dy, dz); });
-        const T curvature = T(3) * (scx + scy + scz);
+        T curvature;
+        if constexpr (sizeof(T) == 8) {
+            curvature = divergence_f64<QQ>(nv);
+        } else {
+            const T scx = lattice_grad<QQ, 0, T>([&](int dx, int dy, int dz) { return nv(0, dx, dy, dz); });
+            const T scy = lattice_grad<QQ, 1, T>([&](int dx, int dy, int dz) { return nv(1, dx, dy, dz); });
+            const T scz = lattice_grad<QQ, 2, T>([&](int dx, int dy, int dz) { return nv(2, dx, dy, dz); });
+            curvature = T(3) * (scx + scy + scz);
+        }
         const T n_x = nv(0, 0, 0, 0), n_y = nv(1, 0, 0, 0), n_z = nv(2, 0, 0, 0), ind = nv(3, 0, 0, 0);
         const T phi = s_phi[z % 3][ty + 2][tx + 2];
         collide_node<QQ, JET, S, MODE>(p, b, x, y, z, t, pop, phi, n_x, n_y, n_z, ind, curvature, s_mlp, col);

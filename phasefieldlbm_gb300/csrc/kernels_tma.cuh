@@ -351,8 +351,14 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
                     auto v = [&](int dx, int dy, int dz) -> T {
                         return phi_at(dz < 0 ? sm : (dz > 0 ? sp : sn), ly + 1 + dy, lx + L::PXO - 1 + dx);
                     };
-                    unit_normal<sizeof(T) == 4>(lattice_grad<QQ, 0, T>(v), lattice_grad<QQ, 1, T>(v),
-                                                lattice_grad<QQ, 2, T>(v), nxv, nyv, nzv, ind);
+                    if constexpr (sizeof(T) == 8) {
+                        T gx, gy, gz;
+                        gradient_f64<QQ>(v, gx, gy, gz);
+                        unit_normal_f64(gx, gy, gz, nxv, nyv, nzv, ind);
+                    } else {
+                        unit_normal<true>(lattice_grad<QQ, 0, T>(v), lattice_grad<QQ, 1, T>(v),
+                                          lattice_grad<QQ, 2, T>(v), nxv, nyv, nzv, ind);
+                    }
                 }
                 n_at(0, nn, ly, lx) = nxv;
                 n_at(1, nn, ly, lx) = nyv;
@@ -415,10 +421,15 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
         auto nv = [&](int c, int dx, int dy, int dz) -> T {
             return n_at(c, dz < 0 ? s_m : (dz > 0 ? s_p : s_0), ty + 1 + dy, tx + 1 + dx);
         };
-        const T scx = lattice_grad<QQ, 0, T>([&](int dx, int dy, int dz) { return nv(0, dx, dy, dz); });
-        const T scy = lattice_grad<QQ, 1, T>([&](int dx, int dy, int dz) { return nv(1, dx, dy, dz); });
-        const T scz = lattice_grad<QQ, 2, T>([&](int dx, int dy, int dz) { return nv(2, dx, dy, dz); });
-        const T curvature = T(3) * (scx + scy + scz);
+        T curvature;
+        if constexpr (sizeof(T) == 8) {
+            curvature = divergence_f64<QQ>(nv);
+        } else {
+            const T scx = lattice_grad<QQ, 0, T>([&](int dx, int dy, int dz) { return nv(0, dx, dy, dz); });
+            const T scy = lattice_grad<QQ, 1, T>([&](int dx, int dy, int dz) { return nv(1, dx, dy, dz); });
+            const T scz = lattice_grad<QQ, 2, T>([&](int dx, int dy, int dz) { return nv(2, dx, dy, dz); });
+            curvature = T(3) * (scx + scy + scz);
+        }
         const T n_x = nv(0, 0, 0, 0), n_y = nv(1, 0, 0, 0), n_z = nv(2, 0, 0, 0), ind = ind_at(z, ty, tx + 1);
         const T phi = phi_at(pslot(z), ty + 2, tx + L::PXO);
 
