@@ -324,6 +324,23 @@ class EngineT final : public Engine {
     dim3 node_block() const { return dim3(32, 8, 1); }
     dim3 node_grid() const { return dim3((h_.nx + 31) / 32, (h_.ny + 7) / 8, h_.nz); }
 
+    // A launch that may begin before the phase kernel in front of it has ended
+    // (the collide kernels wait by themselves, pdl_wait_previous).
+    template <class... P, class... A>
+    static void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A &...args) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, kernel, args...);
+    }
+
     void enqueue_step(int parity, cudaStream_t s, cudaEvent_t *ev) override {
         const StepBuffers<S, T> b = buffers(parity);
         if (ev) cudaEventRecord(ev[0], s);
@@ -332,11 +349,11 @@ class EngineT final : public Engine {
             if constexpr (sizeof(S) >= 4) {
                 const size_t smc = TmaModeLayout<QQ, S, MODE_STEP_CLOSURE>::total + closure_smem_bytes<T>();
                 if (use_tma_ && tma_closure_ && avg_)
-                    k_collide_tma<QQ, JET, S, MODE_STEP_CLOSURE_AVG>
-                        <<<collide_grid(), dim3(TX, TY, 1), smc, s>>>(p_, b, fmapn_[parity], fmapw_[parity], phimap_[parity]);
+                    launch_pdl(k_collide_tma<QQ, JET, S, MODE_STEP_CLOSURE_AVG>, collide_grid(), dim3(TX, TY, 1), smc, s,
+                               p_, b, fmapn_[parity], fmapw_[parity], phimap_[parity]);
                 else if (use_tma_ && tma_closure_)
-                    k_collide_tma<QQ, JET, S, MODE_STEP_CLOSURE>
-                        <<<collide_grid(), dim3(TX, TY, 1), smc, s>>>(p_, b, fmapn_[parity], fmapw_[parity], phimap_[parity]);
+                    launch_pdl(k_collide_tma<QQ, JET, S, MODE_STEP_CLOSURE>, collide_grid(), dim3(TX, TY, 1), smc, s,
+                               p_, b, fmapn_[parity], fmapw_[parity], phimap_[parity]);
                 else if (avg_)
                     k_collide<QQ, JET, S, MODE_STEP_CLOSURE_AVG><<<collide_grid(), dim3(TX, TY, 1), 0, s>>>(p_, b);
                 else
@@ -345,15 +362,15 @@ class EngineT final : public Engine {
         } else if (use_tma_) {
             const size_t sm = TmaLayout<QQ, S>::total;
             if (avg_) {
-                k_collide_tma<QQ, JET, S, MODE_STEP_AVG>
-                    <<<collide_grid(), dim3(TX, TY, 1), sm, s>>>(p_, b, fmapn_[parity], fmapw_[parity], phimap_[parity]);
+                launch_pdl(k_collide_tma<QQ, JET, S, MODE_STEP_AVG>, collide_grid(), dim3(TX, TY, 1), sm, s, p_, b,
+                           fmapn_[parity], fmapw_[parity], phimap_[parity]);
             } else if (use_pair_) {
                 if constexpr (sizeof(T) == 4)
-                    k_collide_pair<QQ, JET, S><<<collide_grid(), dim3(TX2, TY, 1), PairLayout<QQ, S>::total, s>>>(
-                        p_, b, fmapn_[parity], fmapw_[parity], phimap_[parity]);
+                    launch_pdl(k_collide_pair<QQ, JET, S>, collide_grid(), dim3(TX2, TY, 1), PairLayout<QQ, S>::total, s,
+                               p_, b, fmapn_[parity], fmapw_[parity], phimap_[parity]);
             } else {
-                k_collide_tma<QQ, JET, S, MODE_STEP>
-                    <<<collide_grid(), dim3(TX, TY, 1), sm, s>>>(p_, b, fmapn_[parity], fmapw_[parity], phimap_[parity]);
+                launch_pdl(k_collide_tma<QQ, JET, S, MODE_STEP>, collide_grid(), dim3(TX, TY, 1), sm, s, p_, b,
+                           fmapn_[parity], fmapw_[parity], phimap_[parity]);
             }
         } else if (avg_) {
             k_collide<QQ, JET, S, MODE_STEP_AVG><<<collide_grid(), dim3(TX, TY, 1), 0, s>>>(p_, b);

@@ -628,6 +628,7 @@ __global__ void __launch_bounds__(NT2, PairOccupancy<QQ, S>::value)
                    const __grid_constant__ CUtensorMap fmapw, const __grid_constant__ CUtensorMap phimap) {
     extern __shared__ __align__(128) unsigned char smem[];
     tma_pipeline_init<QQ, S, PairLayout<QQ, S>>(smem);
+    pdl_wait_previous();
     const int zb = 1 + blockIdx.z * p.zchunk;
     const int ze = min(zb + p.zchunk, int(p.nz) - 1);
     uint32_t seq = 0;

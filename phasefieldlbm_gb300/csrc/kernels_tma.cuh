@@ -475,6 +475,7 @@ __global__ void __launch_bounds__(NT, CollideOccupancy<QQ, S>::value)
     const int zb = 1 + blockIdx.z * p.zchunk;
     const int ze = min(zb + p.zchunk, int(p.nz) - 1);
     uint32_t seq = 0, tiles = 0;
+    pdl_wait_previous();
     collide_tile_tma<QQ, JET, S, MODE, DefaultTile, L>(p, b, &fmapn, &fmapw, &phimap, int(blockIdx.x) * TX,
                                                        int(blockIdx.y) * TY, zb, ze, smem, seq, tiles, s_mlp);
 }

@@ -8,6 +8,7 @@
 #include "boundary.cuh"
 #include "lattice.cuh"
 #include "params.cuh"
+#include "tma.cuh"
 
 namespace pflbm {
 
@@ -232,6 +233,7 @@ __device__ __forceinline__ void phase_vec4(const Params<float> &p, const StepBuf
 template <int QQ, bool JET, class S>
 __global__ void __launch_bounds__(256, 4)
     k_phase_v4(const __grid_constant__ Params<float> p, const __grid_constant__ StepBuffers<S, float> b) {
+    pdl_release_next();
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const int x4 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
