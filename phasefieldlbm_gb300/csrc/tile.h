@@ -26,31 +26,39 @@ static_assert(kTileX % 32 == 0 && kTileX * kTileY <= 1024, "collide tile");
 // each. Short chunks pay the warm-up of a CTA (four phi planes, two normal
 // planes, an empty pipeline) over and over; the wrong number of chunks leaves
 // most of the chip idle behind a few last CTAs. The time is modelled in planes
-// of a full SM: a wave of full SMs takes the chunk and one plane of warm-up
-// that the neighbours on the SM do not hide; the last, partial wave takes as
-// long on an SM with all its CTAs, three quarters as long with a single one
-// (which has the SM for itself), and hides less (four planes more). The chunk
-// with the least is taken. Against the fastest of a sweep of chunks the choice
-// is 1% slower on average over 22 grids from 32x32x64 to 256x256x1024 (every
-// storage type, plain, averaging and closure kernels; 3% at most) and 2% over
-// 36 random ones (17% at most). Eight CTAs per SM at least four planes long,
-// the rule before, was 10% slower on average over the random ones; us before
-// and after: FP16 256x256x1024 1859 -> 1566; FP32 64x64x128 30.6 -> 24.6;
-// 96^3 46.5 -> 36.3; 128^3 87.1 -> 78.3; 128x128x512 unchanged.
+// of a full SM: a wave of full SMs takes the chunk and one and a half planes
+// of warm-up that the neighbours on the SM do not hide; the last, partial wave
+// takes as long on an SM with all its CTAs, half as long with a single one
+// (which has the SM for itself), and hides less (two planes more). Of the
+// chunks within 6% of the least, the one nearest to 8 planes is taken: what
+// the model calls equal is faster with shorter chunks, whose CTAs read the
+// planes more nearly in order. Against the fastest of a sweep of chunks the
+// choice is 1% slower on average over 22 grids from 32x32x64 to 256x256x1024
+// (every storage type, plain and closure kernels; 4% at most). Eight CTAs per
+// SM at least four planes long, the rule before: FP16 256x256x1024 1859 ->
+// 1494 us, FP32 64x64x128 30.6 -> 22.6, 96^3 46.5 -> 33.1, 128^3 87.1 -> 71.0,
+// of which a fifth to a third is the shorter warm-up.
 inline int pick_zchunk(int tiles, int nzi, int sms, int per_sm) {
-    int best = nzi;
-    double least = 1e300;
-    for (int chunks = 1; chunks <= nzi; ++chunks) {
-        const int zc = (nzi + chunks - 1) / chunks;
-        if (zc < 2 && nzi >= 2) break;
+    auto planes = [&](int chunks) { return (nzi + chunks - 1) / chunks; };
+    auto time = [&](int zc) {
         const long long n = 1ll * tiles * ((nzi + zc - 1) / zc), slots = 1ll * sms * per_sm;
-        double t = double(n / slots) * (zc + 1);
+        double t = double(n / slots) * (zc + 1.5);
         const long long rem = n % slots;
         if (rem > 0) {
             const int on = int((rem + sms - 1) / sms);  // CTAs on the fullest SM
-            t += (per_sm > 1 ? 0.75 + 0.25 * (on - 1) / (per_sm - 1) : 1.0) * (zc + 1) + (on < per_sm ? 4 : 0);
+            t += (per_sm > 1 ? 0.5 + 0.5 * (on - 1) / (per_sm - 1) : 1.0) * (zc + 1.5) + (on < per_sm ? 2 : 0);
         }
-        if (t < least) least = t, best = zc;
+        return t;
+    };
+    double least = 1e300;
+    for (int chunks = 1; chunks <= nzi && (planes(chunks) >= 2 || chunks == 1); ++chunks)
+        least = std::min(least, time(planes(chunks)));
+    int best = nzi;
+    double off = 1e300;
+    for (int chunks = 1; chunks <= nzi && (planes(chunks) >= 2 || chunks == 1); ++chunks) {
+        const int zc = planes(chunks);
+        const double d = zc > 8 ? zc / 8.0 : 8.0 / zc;
+        if (time(zc) <= 1.06 * least && d <= off) off = d, best = zc;
     }
     return std::max(best, 1);
 }
