@@ -48,6 +48,7 @@
 #include "gridbar.cuh"
 #include "kernels.cuh"
 #include "packed.cuh"
+#include "widen.cuh"
 
 namespace {
 
@@ -90,37 +91,73 @@ __host__ __device__ inline uint64_t mix64(uint64_t x) {
 __device__ __forceinline__ float sigmoidf_(float a) { return __frcp_rn(1.0f + expf(-a)); }
 
 // ------------------------------------------------------------- data
-__global__ void k_filter_restrict(const float *__restrict__ macro, uint64_t Nf, int nxf, int nyf, int nzf, int nxc,
-                                  int nyc, int nzc, float *__restrict__ coarse) {
+// Box filter and restriction in FP64, bound by the FP64 unit. A thread owns a
+// coarse column (i, j) of a z chunk, sums every fine plane of its boxes once
+// and carries plane 2k+1 on to the next coarse plane; the floats are widened on
+// the integer units: 251 FP64 instructions per coarse node instead of 455 with
+// the conversions, 64x64x256 coarse nodes 910 -> 560 us (753 with the
+// conversions in FP64).
+constexpr int kFilterX = 32, kFilterY = 4, kFilterPlanes = 8;
+__global__ void __launch_bounds__(kFilterX *kFilterY) k_filter_restrict(const float *__restrict__ macro, uint64_t Nf,
+                                                                        int nxf, int nyf, int nzf, int nxc, int nyc,
+                                                                        int nzc, float *__restrict__ coarse) {
     const uint64_t Nc = uint64_t(nxc) * nyc * nzc;
-    for (uint64_t c = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; c < Nc; c += uint64_t(gridDim.x) * blockDim.x) {
-        const int i = int(c % nxc), j = int((c / nxc) % nyc), k = int(c / (uint64_t(nxc) * nyc));
-        double s[11] = {0};
-        for (int dz = -1; dz <= 1; ++dz)
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dx = -1; dx <= 1; ++dx) {
-                    const int X = min(max(2 * i + dx, 0), nxf - 1), Y = min(max(2 * j + dy, 0), nyf - 1),
-                              Z = min(max(2 * k + dz, 0), nzf - 1);
-                    const uint64_t f = uint64_t(X) + uint64_t(nxf) * (uint64_t(Y) + uint64_t(nyf) * Z);
-                    const double r = macro[pflbm::M_RHO * Nf + f], ux = macro[pflbm::M_UX * Nf + f],
-                                 uy = macro[pflbm::M_UY * Nf + f], uz = macro[pflbm::M_UZ * Nf + f],
-                                 ph = macro[pflbm::M_PHI * Nf + f];
-                    s[0] += r; s[1] += ux; s[2] += uy; s[3] += uz; s[4] += ph;
-                    s[5] += ux * ux; s[6] += uy * uy; s[7] += uz * uz;
-                    s[8] += ux * uy; s[9] += ux * uz; s[10] += uy * uz;
-                }
-        for (int q = 0; q < 11; ++q) s[q] *= 1.0 / 27.0;
-        coarse[0 * Nc + c] = float(s[0]);
-        coarse[1 * Nc + c] = float(s[1]);
-        coarse[2 * Nc + c] = float(s[2]);
-        coarse[3 * Nc + c] = float(s[3]);
-        coarse[4 * Nc + c] = float(s[4]);
-        coarse[5 * Nc + c] = float(s[5] - s[1] * s[1]);
-        coarse[6 * Nc + c] = float(s[6] - s[2] * s[2]);
-        coarse[7 * Nc + c] = float(s[7] - s[3] * s[3]);
-        coarse[8 * Nc + c] = float(s[8] - s[1] * s[2]);
-        coarse[9 * Nc + c] = float(s[9] - s[1] * s[3]);
-        coarse[10 * Nc + c] = float(s[10] - s[2] * s[3]);
+    const int i = int(blockIdx.x) * kFilterX + threadIdx.x, j = int(blockIdx.y) * kFilterY + threadIdx.y;
+    if (i >= nxc || j >= nyc) return;
+    const int xm = max(2 * i - 1, 0), x0 = min(2 * i, nxf - 1), xp = min(2 * i + 1, nxf - 1);
+    const int slot[5] = {pflbm::M_RHO, pflbm::M_UX, pflbm::M_UY, pflbm::M_UZ, pflbm::M_PHI};
+    // sums over the x triple of fine row y, plane z
+    auto row = [&](int y, int z, double (&r)[kCoarseFields]) {
+        const uint64_t base = uint64_t(nxf) * (uint64_t(min(max(y, 0), nyf - 1)) + uint64_t(nyf) * z);
+        float q[15];
+        double v[15];
+#pragma unroll
+        for (int f = 0; f < 5; ++f) {
+            const float *p = macro + slot[f] * Nf + base;
+            q[3 * f] = p[xm], q[3 * f + 1] = p[x0], q[3 * f + 2] = p[xp];
+        }
+        pflbm::widen_all(q, v);
+#pragma unroll
+        for (int f = 0; f < 5; ++f) r[f] = v[3 * f] + v[3 * f + 1] + v[3 * f + 2];
+        constexpr int A[6] = {1, 2, 3, 1, 1, 2}, B[6] = {1, 2, 3, 2, 3, 3};
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            r[5 + k] = fma(v[3 * A[k] + 2], v[3 * B[k] + 2],
+                           fma(v[3 * A[k] + 1], v[3 * B[k] + 1], v[3 * A[k]] * v[3 * B[k]]));
+    };
+    // sums over the three rows of the box in fine plane z (clamped)
+    auto plane = [&](int z, double (&s)[kCoarseFields]) {
+        z = min(max(z, 0), nzf - 1);
+        double r[kCoarseFields];
+        row(2 * j, z, s);
+#pragma unroll
+        for (int dy = -1; dy <= 1; dy += 2) {
+            row(2 * j + dy, z, r);
+#pragma unroll
+            for (int f = 0; f < kCoarseFields; ++f) s[f] += r[f];
+        }
+    };
+    const int k0 = int(blockIdx.z) * kFilterPlanes, k1 = min(k0 + kFilterPlanes, nzc);
+    double below[kCoarseFields], s[kCoarseFields], above[kCoarseFields];
+    plane(2 * k0 - 1, below);
+    for (int k = k0; k < k1; ++k) {
+        plane(2 * k, s);
+        plane(2 * k + 1, above);
+        double m[kCoarseFields];
+#pragma unroll
+        for (int f = 0; f < kCoarseFields; ++f) {
+            m[f] = (below[f] + s[f] + above[f]) * (1.0 / 27.0);
+            below[f] = above[f];
+        }
+        const uint64_t c = uint64_t(i) + uint64_t(nxc) * (uint64_t(j) + uint64_t(nyc) * k);
+#pragma unroll
+        for (int f = 0; f < 5; ++f) coarse[f * Nc + c] = float(m[f]);
+        coarse[5 * Nc + c] = float(m[5] - m[1] * m[1]);
+        coarse[6 * Nc + c] = float(m[6] - m[2] * m[2]);
+        coarse[7 * Nc + c] = float(m[7] - m[3] * m[3]);
+        coarse[8 * Nc + c] = float(m[8] - m[1] * m[2]);
+        coarse[9 * Nc + c] = float(m[9] - m[1] * m[3]);
+        coarse[10 * Nc + c] = float(m[10] - m[2] * m[3]);
     }
 }
 
@@ -1086,8 +1123,10 @@ int pflbm_closure_add_snapshot(pflbm_closure *c, pflbm_sim *fine, int32_t stride
         return fail(PFLBM_ERR_INVALID_ARG, "closure sample capacity exceeded (" + std::to_string(c->n + count) + " > " +
                                                std::to_string(c->cap) + ")");
     // the fine run's analysis ran on its own stream, which sim_view synchronised
-    k_filter_restrict<<<1216, 256, 0, c->stream>>>(static_cast<const float *>(v.macro), v.N, int(v.nx), int(v.ny),
-                                                   int(v.nz), nxc, nyc, nzc, c->coarse);
+    const dim3 fg((nxc + kFilterX - 1) / kFilterX, (nyc + kFilterY - 1) / kFilterY,
+                  (nzc + kFilterPlanes - 1) / kFilterPlanes);
+    k_filter_restrict<<<fg, dim3(kFilterX, kFilterY), 0, c->stream>>>(
+        static_cast<const float *>(v.macro), v.N, int(v.nx), int(v.ny), int(v.nz), nxc, nyc, nzc, c->coarse);
     k_make_samples<<<kMakeBlocks, kMakeThreads, 0, c->stream>>>(
         c->coarse, nxc, nyc, nzc, stride, float(v.tau_water), float(v.tau_oil), i0, ni, j0, nj, c->X, c->Y, c->n,
         static_cast<const float *>(v.macro), v.N, int(v.nx), int(v.ny), c->width_part);

@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "widen.cuh"
+
 namespace pflbm {
 
 constexpr int RED_FIELDS = 12;  // phi, rho, rho ux, rho uy, rho uz, max |u|^2, rho_in, n_in, rho_out, n_out, nonfinite, spare
@@ -14,8 +16,8 @@ constexpr int RED_MAX_SLOT = 5; // max |u|^2 (combined by max; every other slot 
 // float fields are classified as floats (phi > 0.9 and phi < 0.1 select the
 // same floats against 0.9f and 0.1f), and the square root is taken of the
 // largest |u|^2 only, which gives the largest root (the root is monotone).
-// With the 64-bit divisions per node gone as well, 128^3 nodes and the final
-// pass: 222 -> 84 us.
+// Floats are widened on the integer units. With the 64-bit divisions per node
+// gone as well, 128^3 nodes and the final pass: 222 -> 73 us.
 struct RedAcc {
     double phi = 0.0, rho = 0.0, mx = 0.0, my = 0.0, mz = 0.0, u2 = 0.0, rho_in = 0.0, rho_out = 0.0;
     unsigned int n_in = 0u, n_out = 0u, bad = 0u;
@@ -26,8 +28,16 @@ struct RedAcc {
             ++bad;
             return;
         }
-        const double dr = r, dx = ux, dy = uy, dz = uz;
-        phi += double(p);
+        const T in[5] = {r, ux, uy, uz, p};
+        double wide[5];
+        if constexpr (sizeof(T) == 4) {
+            widen_all(in, wide);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 5; ++k) wide[k] = in[k];
+        }
+        const double dr = wide[0], dx = wide[1], dy = wide[2], dz = wide[3];
+        phi += wide[4];
         rho += dr;
         mx = fma(dr, dx, mx);
         my = fma(dr, dy, my);
@@ -86,7 +96,7 @@ __device__ __forceinline__ void block_reduce_row(double (&acc)[RED_FIELDS], doub
 
 // The total of `n` rows in slot f, by the calling warp (lane-strided, then a
 // shuffle tree; lane 0 has it); the max slot becomes max |u|. One thread per
-// slot took 71 us for 608 rows.
+// slot took 71 us for 608 rows, a warp per slot takes 9.
 constexpr int RED_FINAL_THREADS = 32 * RED_FIELDS;
 __device__ __forceinline__ double red_total(const double *rows, int n, int f) {
     double s = 0.0;
