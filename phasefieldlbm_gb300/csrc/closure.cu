@@ -384,22 +384,25 @@ __global__ void __launch_bounds__(kSB) k_mlp_grad(const float *__restrict__ blob
 // weights are laid out once as TF32 fragments in lane order (8-byte
 // conflict-free loads instead of 4- and 8-way conflicts and a conversion per
 // use), a sigmoid is evaluated once per unit instead of two or three times,
-// and two warps share what one warp did: 2^20 samples 398 -> 226 us (IPC 1.6
-// at 16 warps per SM; 3640 warp instructions per 32 samples).
+// and two warps share what one warp did: 2^20 samples 398 -> 226 us at 16
+// warps per SM (IPC 1.6, 3640 warp instructions per 32 samples), 202 us at 24.
 constexpr int kTcThreads = 2 * kSB;
 constexpr int kTcPairs = kSB / 32;
 constexpr int kTcX = 12;         // row stride of the Xn tile (words)
 constexpr int kTcH = kMlpH + 4;  // row stride of the 32-wide tiles
 // shared words: weight fragments and constants, then per pair Xn, H1 (TF32
-// bits), dA2, dA1, dz, loss, the w3 sums of the first tile, then the pairs'
-// partial gradients
-constexpr int kTcF1 = 0, kTcF2 = kTcF1 + 256, kTcF2T = kTcF2 + 1024, kTcB1 = kTcF2T + 1024, kTcB2 = kTcB1 + kMlpH,
+// bits), dA2, dA1 (each first holding SiLU' of its units), dz, loss, the w3
+// sums of the first tile; the pair's partial gradient takes the same place
+// when the tiles have been read. With that, and W2's fragments read as scalars
+// for the transposed product, three CTAs fit an SM (72 KB, 80 registers)
+constexpr int kTcF1 = 0, kTcF2 = kTcF1 + 256, kTcB1 = kTcF2 + 1024, kTcB2 = kTcB1 + kMlpH,
               kTcW3 = kTcB2 + kMlpH, kTcMean = kTcW3 + kMlpH, kTcInv = kTcMean + kMlpIn, kTcB3 = kTcInv + kMlpIn,
               kTcScale = kTcB3 + 1, kTcWeights = kTcB3 + 4;
 constexpr int kTcPairWords = 32 * kTcX + 3 * 32 * kTcH + 32 + 32 + 8 * 32;
 constexpr int kTcPart = kMlpParams + 1;  // partial gradient + loss
 constexpr int kTcAcc = (kTcPart + kTcThreads - 1) / kTcThreads;  // FP64 sums per thread
-constexpr int kTcSmem = 4 * (kTcWeights + kTcPairs * kTcPairWords + kTcPairs * kTcPart);
+constexpr int kTcSmem = 4 * (kTcWeights + kTcPairs * kTcPairWords);
+static_assert(kTcPart <= kTcPairWords, "the partial gradient takes the pair's tiles' place");
 static_assert(kMlpH == 32 && kMlpIn == 8, "fragment layout");
 
 __device__ __forceinline__ uint32_t to_tf32(float x) {
@@ -421,8 +424,7 @@ __device__ __forceinline__ void mma_tf32_1688(float (&d)[4], const uint32_t (&a)
 __device__ __forceinline__ void pair_sync(int pair) { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); }
 
 // The blob as fragments: B operand words of lane (g = lane / 4, t = lane % 4)
-// side by side, W1 and W2 by output column block and k step, W2 once more
-// transposed for the backward product. Read past the L1, which another CTA's
+// side by side, W1 and W2 by output column block and k step. Read past the L1, which another CTA's
 // update of the blob does not invalidate.
 __device__ __forceinline__ void tc_load_weights(float *s, const float *blob) {
     uint32_t *w = reinterpret_cast<uint32_t *>(s);
@@ -442,9 +444,7 @@ __device__ __forceinline__ void tc_load_weights(float *s, const float *blob) {
             s[kTcB1 + i - pflbm::kMlpB1] = v;
         } else if (i < pflbm::kMlpB2) {
             const int j = (i - pflbm::kMlpW2) >> 5, c = (i - pflbm::kMlpW2) & 31;
-            const uint32_t b = to_tf32(v);
-            w[kTcF2 + (((j >> 3) * 4 + (c >> 3)) * 32 + (j & 7) * 4 + (c & 3)) * 2 + ((c >> 2) & 1)] = b;
-            w[kTcF2T + (((c >> 3) * 4 + (j >> 3)) * 32 + (c & 7) * 4 + (j & 3)) * 2 + ((j >> 2) & 1)] = b;
+            w[kTcF2 + (((j >> 3) * 4 + (c >> 3)) * 32 + (j & 7) * 4 + (c & 3)) * 2 + ((c >> 2) & 1)] = to_tf32(v);
         } else if (i < pflbm::kMlpW3) {
             s[kTcB2 + i - pflbm::kMlpB2] = v;
         } else if (i < pflbm::kMlpB3) {
@@ -497,9 +497,10 @@ __device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&
     float *dzs = da1s + 32 * kTcH;                      // [32]
     float *losses = dzs + 32;                           // [32]
     float *w3p = losses + 32;                           // [8][32]
-    float *part = s + kTcWeights + kTcPairs * kTcPairWords + pair * kTcPart;
-    const uint2 *f1 = reinterpret_cast<const uint2 *>(s + kTcF1), *f2 = reinterpret_cast<const uint2 *>(s + kTcF2),
-                *f2t = reinterpret_cast<const uint2 *>(s + kTcF2T);
+    float *part = base;
+    const uint2 *f1 = reinterpret_cast<const uint2 *>(s + kTcF1), *f2 = reinterpret_cast<const uint2 *>(s + kTcF2);
+    // W2[8 kk + t (+4)][8 nt + g]: the word of lane (g, t) in the transposed product
+    const uint32_t *f2t = reinterpret_cast<const uint32_t *>(s + kTcF2) + (t * 4 + (g & 3)) * 2 + (g >> 2);
 
     // normalised features
     {
@@ -516,8 +517,7 @@ __device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&
     __syncwarp();
 
     const int r0 = 16 * half + g;  // fragment rows r0 and r0 + 8, columns 8 nt + 2 t (+1)
-    // layer 1: a1 = Xn W1^T + b1; h1 = SiLU(a1) to shared memory, SiLU'(a1) kept
-    float sg1[4][4];
+    // layer 1: a1 = Xn W1^T + b1; h1 = SiLU(a1) and SiLU'(a1) to shared memory
     {
         const uint32_t a[4] = {xs[r0 * kTcX + t], xs[(r0 + 8) * kTcX + t], xs[r0 * kTcX + t + 4],
                                xs[(r0 + 8) * kTcX + t + 4]};
@@ -529,14 +529,15 @@ __device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float sg = sigmoidf_(d[e]);
-                h1s[(r0 + (e >= 2 ? 8 : 0)) * kTcH + 8 * nt + 2 * t + (e & 1)] = to_tf32(d[e] * sg);
-                sg1[nt][e] = sg * (1.0f + d[e] * (1.0f - sg));
+                const int at = (r0 + (e >= 2 ? 8 : 0)) * kTcH + 8 * nt + 2 * t + (e & 1);
+                h1s[at] = to_tf32(d[e] * sg);
+                da1s[at] = sg * (1.0f + d[e] * (1.0f - sg));
             }
         }
     }
     __syncwarp();
     // layer 2: a2 = H1 W2^T + b2; z = w3 . SiLU(a2) + b3 per sample
-    float h2[4][4], sg2[4][4], zp[2] = {0.f, 0.f};
+    float h2[4][4], zp[2] = {0.f, 0.f};
     {
         uint32_t a[4][4];
 #pragma unroll
@@ -556,7 +557,7 @@ __device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&
             for (int e = 0; e < 4; ++e) {
                 const float sg = sigmoidf_(d[e]);
                 h2[nt][e] = d[e] * sg;
-                sg2[nt][e] = sg * (1.0f + d[e] * (1.0f - sg));
+                da2s[(r0 + (e >= 2 ? 8 : 0)) * kTcH + 8 * nt + 2 * t + (e & 1)] = sg * (1.0f + d[e] * (1.0f - sg));
                 zp[e >> 1] = __fmaf_rn(s[kTcW3 + 8 * nt + 2 * t + (e & 1)], h2[nt][e], zp[e >> 1]);
             }
         }
@@ -587,8 +588,8 @@ __device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int col = 8 * nt + 2 * t + (e & 1);
-            da2s[(r0 + (e >= 2 ? 8 : 0)) * kTcH + col] = (e >= 2 ? dz1 : dz0) * s[kTcW3 + col] * sg2[nt][e];
+            const int col = 8 * nt + 2 * t + (e & 1), at = (r0 + (e >= 2 ? 8 : 0)) * kTcH + col;
+            da2s[at] = (e >= 2 ? dz1 : dz0) * s[kTcW3 + col] * da2s[at];
         }
     if (half == 0) {
 #pragma unroll
@@ -610,15 +611,19 @@ __device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&
         for (int nt = 0; nt < 4; ++nt) {
             float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) mma_tf32_1688(d, a[kk], f2t[(nt * 4 + kk) * 32 + lane]);
+            for (int kk = 0; kk < 4; ++kk)
+                mma_tf32_1688(d, a[kk], make_uint2(f2t[(kk * 4 + nt) * 64], f2t[(kk * 4 + nt) * 64 + 32]));
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                da1s[(r0 + (e >= 2 ? 8 : 0)) * kTcH + 8 * nt + 2 * t + (e & 1)] = d[e] * sg1[nt][e];
+            for (int e = 0; e < 4; ++e) {
+                const int at = (r0 + (e >= 2 ? 8 : 0)) * kTcH + 8 * nt + 2 * t + (e & 1);
+                da1s[at] = d[e] * da1s[at];
+            }
         }
     }
     pair_sync(pair);
     // weight gradients over the pair's 32 samples (K): this warp the output
     // rows 16 half .. 16 half + 15
+    float dw2[4][4], dw1[4] = {0.f, 0.f, 0.f, 0.f};
     {
         uint32_t a[4][4];
 #pragma unroll
@@ -630,46 +635,35 @@ __device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&
         }
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {  // dW2[j][i] = sum_s dA2[s][j] H1[s][i]
-            float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dw2[nt][e] = 0.f;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                mma_tf32_1688(d, a[kk], make_uint2(h1s[(8 * kk + t) * kTcH + 8 * nt + g],
-                                                   h1s[(8 * kk + t + 4) * kTcH + 8 * nt + g]));
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                part[pflbm::kMlpW2 + (r0 + (e >= 2 ? 8 : 0)) * kMlpH + 8 * nt + 2 * t + (e & 1)] = d[e];
+                mma_tf32_1688(dw2[nt], a[kk], make_uint2(h1s[(8 * kk + t) * kTcH + 8 * nt + g],
+                                                         h1s[(8 * kk + t + 4) * kTcH + 8 * nt + g]));
         }
-        float d[4] = {0.f, 0.f, 0.f, 0.f};  // dW1[i][q] = sum_s dA1[s][i] Xn[s][q]
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
+        for (int kk = 0; kk < 4; ++kk) {  // dW1[i][q] = sum_s dA1[s][i] Xn[s][q]
             const uint32_t b[4] = {to_tf32(da1s[(8 * kk + t) * kTcH + r0]), to_tf32(da1s[(8 * kk + t) * kTcH + r0 + 8]),
                                    to_tf32(da1s[(8 * kk + t + 4) * kTcH + r0]),
                                    to_tf32(da1s[(8 * kk + t + 4) * kTcH + r0 + 8])};
-            mma_tf32_1688(d, b, make_uint2(xs[(8 * kk + t) * kTcX + g], xs[(8 * kk + t + 4) * kTcX + g]));
+            mma_tf32_1688(dw1, b, make_uint2(xs[(8 * kk + t) * kTcX + g], xs[(8 * kk + t + 4) * kTcX + g]));
         }
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            part[pflbm::kMlpW1 + (r0 + (e >= 2 ? 8 : 0)) * kMlpIn + 2 * t + (e & 1)] = d[e];
     }
     // bias gradients: column sums over the pair's samples, b1 by the first
-    // warp, b2 by the second
+    // warp, b2 by the second; b3 and the loss by the first, w3 by the second
+    float sb = 0.f, sdz = 0.f, sl = 0.f, dw3[8];
     {
         const float *col = (half == 0 ? da1s : da2s) + lane;
-        float sum = 0.f;
 #pragma unroll
-        for (int r = 0; r < 32; ++r) sum += col[r * kTcH];
-        part[(half == 0 ? pflbm::kMlpB1 : pflbm::kMlpB2) + lane] = sum;
+        for (int r = 0; r < 32; ++r) sb += col[r * kTcH];
     }
     if (half == 0) {
-        float sdz = dzs[lane], sl = losses[lane];
+        sdz = dzs[lane], sl = losses[lane];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             sdz += __shfl_xor_sync(0xffffffffu, sdz, o);
             sl += __shfl_xor_sync(0xffffffffu, sl, o);
-        }
-        if (lane == 0) {
-            part[pflbm::kMlpB3] = sdz;
-            part[kMlpParams] = sl;
         }
     } else {
 #pragma unroll
@@ -679,19 +673,37 @@ __device__ __forceinline__ void tc_block(float *s, const TcRows &rows, double (&
             v += __shfl_xor_sync(0xffffffffu, v, 4);
             v += __shfl_xor_sync(0xffffffffu, v, 8);
             v += __shfl_xor_sync(0xffffffffu, v, 16);
-            if (g == 0) part[pflbm::kMlpW3 + 8 * (k >> 1) + 2 * t + (k & 1)] = v;
+            dw3[k] = v;
         }
+    }
+    pair_sync(pair);  // the tiles have been read
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            part[pflbm::kMlpW2 + (r0 + (e >= 2 ? 8 : 0)) * kMlpH + 8 * nt + 2 * t + (e & 1)] = dw2[nt][e];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        part[pflbm::kMlpW1 + (r0 + (e >= 2 ? 8 : 0)) * kMlpIn + 2 * t + (e & 1)] = dw1[e];
+    part[(half == 0 ? pflbm::kMlpB1 : pflbm::kMlpB2) + lane] = sb;
+    if (half == 0 && lane == 0) {
+        part[pflbm::kMlpB3] = sdz;
+        part[kMlpParams] = sl;
+    }
+    if (half == 1 && g == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) part[pflbm::kMlpW3 + 8 * (k >> 1) + 2 * t + (k & 1)] = dw3[k];
     }
     __syncthreads();
     // the block's sums, pairs in order
-    const float *parts = s + kTcWeights + kTcPairs * kTcPairWords;
+    const float *parts = s + kTcWeights;
 #pragma unroll
     for (int j = 0; j < kTcAcc; ++j) {
         const int p = threadIdx.x + kTcThreads * j;
         if (p <= kMlpParams) {
             float v = 0.0f;
 #pragma unroll
-            for (int q = 0; q < kTcPairs; ++q) v += parts[q * kTcPart + p];
+            for (int q = 0; q < kTcPairs; ++q) v += parts[q * kTcPairWords + p];
             acc[j] += v;
         }
     }
@@ -729,7 +741,7 @@ __device__ __forceinline__ double tc_sum_rows(const double *gsum, int rows, int 
 
 // Gradient of the first `count` samples: every CTA runs its share of the
 // blocks and writes its FP64 sums as a row of gsum; k_grad_rows adds the rows.
-__global__ void __launch_bounds__(kTcThreads, 2) k_mlp_grad_tc(const float *__restrict__ blob,
+__global__ void __launch_bounds__(kTcThreads, 3) k_mlp_grad_tc(const float *__restrict__ blob,
                                                                const float *__restrict__ X,
                                                                const float *__restrict__ Y, uint64_t n,
                                                                uint64_t count, int blocks, double *__restrict__ gsum) {
@@ -774,8 +786,8 @@ __device__ __forceinline__ void adam_update(float g, float lr, float beta1, floa
 // that the CTA owns (moments in registers), grid barrier, the new blob as
 // fragments. The next iteration's samples do not depend on the parameters and
 // are fetched while the CTA waits at the first barrier. 16 384 samples per iteration: 36 us
-// (two launches) -> 13 us: the block 6.1, its FP64 row and the sums 2.5, the
-// barriers 3, the weights 0.8.
+// (two launches) -> 11.7 us, about half of it the block, the rest its FP64 row,
+// the sums, the barriers and the weights.
 constexpr int kTrainChunk = 128;  // iterations per launch
 struct TrainArgs {
     float *blob, *m, *v;
@@ -950,7 +962,7 @@ struct pflbm_closure {
     float *gpart = nullptr;  // per-block gradients of the CUDA-core kernel
     int gpart_blocks = 0;
     double *gsum = nullptr;  // per-CTA gradient sums of the tensor-core kernels
-    int grad_ctas = 0;       // resident CTAs of the tensor-core kernels: rows of gsum
+    int grad_ctas = 0, train_ctas = 0;  // resident CTAs of the gradient and the training kernel
     unsigned int *sync = nullptr;  // grid barrier count and error word of the training kernel
     double *grad = nullptr, *partial = nullptr, *loss_log = nullptr;
     int loss_log_cap = 0;
@@ -1016,7 +1028,7 @@ void launch_grad_simt(pflbm_closure *c, int blocks, int mode, uint64_t seed, uin
 // one CTA per block as far as they are all resident, and never fewer than
 // own all parameters.
 cudaError_t launch_train(pflbm_closure *c, TrainArgs &a) {
-    const int grid = std::max(kSumCtas, std::min(a.blocks, c->grad_ctas));
+    const int grid = std::max(kSumCtas, std::min(a.blocks, c->train_ctas));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kTcThreads);
@@ -1068,13 +1080,15 @@ int pflbm_closure_create(int32_t device, uint64_t max_samples, pflbm_closure **o
         cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
         return cuda_fail(cudaGetLastError(), "gradient kernel shared memory");
     // both kernels run at most as many CTAs as are resident at once
-    int sms = 0, per_sm = 0;
+    int sms = 0, grad = 0, train = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mlp_train, kTcThreads, kTcSmem) != cudaSuccess ||
-        sms * per_sm < kSumCtas)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&grad, k_mlp_grad_tc, kTcThreads, kTcSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&train, k_mlp_train, kTcThreads, kTcSmem) != cudaSuccess ||
+        grad < 1 || sms * train < kSumCtas)
         return cuda_fail(cudaGetLastError(), "training kernel occupancy");
-    c->grad_ctas = sms * per_sm;
-    if (cudaMalloc(&c->gsum, sizeof(double) * size_t(c->grad_ctas) * kTcPart) != cudaSuccess) {
+    c->grad_ctas = sms * grad;
+    c->train_ctas = sms * train;
+    if (cudaMalloc(&c->gsum, sizeof(double) * size_t(std::max(c->grad_ctas, c->train_ctas)) * kTcPart) != cudaSuccess) {
         cudaGetLastError();
         return fail(PFLBM_ERR_OUT_OF_MEMORY, "closure buffers");
     }
