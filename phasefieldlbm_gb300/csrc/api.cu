@@ -4,7 +4,7 @@
 // The time loop of src/main.cu:163-188 launches a captured graph and two
 // boundary kernels and synchronises the host every step. Here one step is
 // two kernels (boundary conditions are folded into them) and whole chunks of
-// steps are captured into one graph, so a run of n steps costs n/16 graph
+// steps are captured into one graph, so a run of n steps costs about n/16 graph
 // launches and no host synchronisation until the caller asks for one.
 #include <cuda_runtime.h>
 
@@ -56,7 +56,7 @@ int cuda_fail(cudaError_t e, const char *what) {
     return fail(PFLBM_ERR_CUDA, m);
 }
 
-constexpr int kChunk = 16;  // steps per captured graph
+constexpr int kChunks[2] = {16, 8};  // steps per captured graph
 
 const char *kFieldNames[PFLBM_FIELD_COUNT] = {
     "rho", "ux", "uy", "uz", "pxx", "pyy", "pzz", "pxy", "pxz", "pyz", "phi", "normx", "normy", "normz", "ind",
@@ -71,8 +71,8 @@ struct pflbm_sim {
     int device = 0;
     std::unique_ptr<Engine> eng;
     cudaStream_t stream = nullptr;
-    // graphs[parity][0] = 1 step, [1] = 2 steps, [2] = kChunk steps
-    cudaGraphExec_t graphs[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
+    cudaGraphExec_t graphs[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // by parity: kChunks[k] steps
+    unsigned int *host_err = nullptr;  // page-locked copy of the device error word
     int parity = 0;          // ping-pong buffer read by the next step
     uint64_t step = 0;       // completed steps
     bool initialized = false;
@@ -223,11 +223,22 @@ int capture(pflbm_sim *s, int parity, int nsteps, cudaGraphExec_t *out) {
     return PFLBM_OK;
 }
 
-// Reads the device error word (set by a kernel whose bounded wait gave up).
-int check_device_error(pflbm_sim *s) {
-    unsigned int w = 0;
-    cudaError_t e = cudaMemcpy(&w, s->eng->error_word(), sizeof w, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, "error word readback");
+int capture_graphs(pflbm_sim *s) {
+    for (int par = 0; par < 2; ++par)
+        for (int k = 0; k < 2; ++k)
+            if (const int rc = capture(s, par, kChunks[k], &s->graphs[par][k])) return rc;
+    return PFLBM_OK;
+}
+
+// Waits for the stream and reads the device error word (set by a kernel whose
+// bounded wait gave up), copied behind the work it reports on: one wait
+// instead of a wait and a blocking copy.
+int synchronize(pflbm_sim *s) {
+    cudaError_t e = cudaMemcpyAsync(s->host_err, s->eng->error_word(), sizeof *s->host_err, cudaMemcpyDeviceToHost,
+                                    s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
+    const unsigned int w = *s->host_err;
     if (w != 0) return fail(PFLBM_ERR_DEVICE, "a kernel gave up waiting for its TMA copies (error word " + std::to_string(w) + ")");
     return PFLBM_OK;
 }
@@ -246,25 +257,32 @@ bool base_field(int32_t id) {
            id == PFLBM_FIELD_PHI || id == PFLBM_FIELD_IND;
 }
 
+// Enqueues what brings the cache up to date; its readers follow on the stream.
 int ensure_cache(pflbm_sim *s, bool full = false) {
     if (full) s->wants_full = true;
     // at step 0 the cache still holds the initial fields
     if (s->cache_step == int64_t(s->step) && (s->cache_full || !full)) return PFLBM_OK;
+    cudaGetLastError();  // an earlier call's error is not this launch's
     s->eng->enqueue_analysis(s->parity ^ 1, uint32_t(s->step - 1), s->wants_full, s->stream);
     s->eng->enqueue_vorticity(s->stream);
-    cudaError_t e = cudaStreamSynchronize(s->stream);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "analysis");
     s->cache_step = int64_t(s->step);
     s->cache_full = s->wants_full;
     return PFLBM_OK;
 }
 
-// Copies real-typed device data to host doubles or floats.
+// Copies real-typed device data to host doubles or floats, behind the work on
+// the stream.
 int copy_out(pflbm_sim *s, const void *dev, size_t n, void *host, bool as_double) {
     const int rb = s->eng->real_bytes();
+    auto copy = [&](void *to) -> cudaError_t {
+        const cudaError_t e = cudaMemcpyAsync(to, dev, n * rb, cudaMemcpyDeviceToHost, s->stream);
+        return e == cudaSuccess ? cudaStreamSynchronize(s->stream) : e;
+    };
     cudaError_t e;
     if ((rb == 4 && !as_double) || (rb == 8 && as_double)) {
-        e = cudaMemcpy(host, dev, n * rb, cudaMemcpyDeviceToHost);
+        e = copy(host);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy D2H");
         return PFLBM_OK;
     }
@@ -272,7 +290,7 @@ int copy_out(pflbm_sim *s, const void *dev, size_t n, void *host, bool as_double
     // cross the C ABI
     std::unique_ptr<unsigned char[]> tmp(new (std::nothrow) unsigned char[n * rb]);
     if (!tmp) return fail(PFLBM_ERR_OUT_OF_MEMORY, "host conversion buffer");
-    e = cudaMemcpy(tmp.get(), dev, n * rb, cudaMemcpyDeviceToHost);
+    e = copy(tmp.get());
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy D2H");
     if (rb == 4) {
         const float *src = reinterpret_cast<const float *>(tmp.get());
@@ -352,6 +370,9 @@ int sim_view(pflbm_sim *s, SimView &v) {
     flush_initial(s);
     int rc = ensure_cache(s);
     if (rc) return rc;
+    // the caller reads on a stream of its own
+    const cudaError_t e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "analysis");
     v.macro = s->eng->macro_ptr();
     v.real_bytes = s->eng->real_bytes();
     v.nx = s->hp.nx;
@@ -433,6 +454,8 @@ void release_resources(pflbm_sim *s) {
     if (s->writer.joinable()) s->writer.join();
     free_pinned(s);
     destroy_graphs(s);
+    if (s->host_err) cudaFreeHost(s->host_err);
+    s->host_err = nullptr;
     if (s->dev_diag) cudaFree(s->dev_diag);
     s->dev_diag = nullptr;
     s->eng.reset();
@@ -536,12 +559,12 @@ int pflbm_create(const pflbm_config *cfg, pflbm_sim **out) {
     if (e != cudaSuccess) return abandon(cuda_fail(e, "cudaStreamCreate"));
     e = cudaMalloc(&s->dev_diag, sizeof(double) * 16);
     if (e != cudaSuccess) return abandon(cuda_fail(e, "cudaMalloc diag"));
-    const int counts[3] = {1, 2, kChunk};
-    for (int par = 0; par < 2; ++par)
-        for (int k = 0; k < 3; ++k) {
-            rc = capture(s.get(), par, counts[k], &s->graphs[par][k]);
-            if (rc) return abandon(rc);
-        }
+    if (cudaMallocHost(&s->host_err, sizeof *s->host_err) != cudaSuccess) {
+        cudaGetLastError();
+        return abandon(fail(PFLBM_ERR_OUT_OF_MEMORY, "cudaMallocHost (error word)"));
+    }
+    rc = capture_graphs(s.get());
+    if (rc) return abandon(rc);
     *out = s.release();
     return PFLBM_OK;
 }
@@ -597,27 +620,30 @@ int pflbm_step_async(pflbm_sim *s, uint64_t n) {
     cudaSetDevice(s->device);
     flush_initial(s);
     uint64_t left = n;
-    while (left > 0) {
-        int k;
-        if (left >= uint64_t(kChunk)) k = 2;
-        else if (left >= 2) k = 1;
-        else k = 0;
-        const int steps = k == 2 ? kChunk : (k == 1 ? 2 : 1);
-        cudaError_t e = cudaGraphLaunch(s->graphs[s->parity][k], s->stream);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
-        if (steps & 1) s->parity ^= 1;
-        s->step += steps;
-        left -= steps;
+    for (int k = 0; k < 2; ++k)
+        for (; left >= uint64_t(kChunks[k]); left -= kChunks[k]) {
+            const cudaError_t e = cudaGraphLaunch(s->graphs[s->parity][k], s->stream);
+            if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
+            s->step += kChunks[k];
+        }
+    // the remaining steps kernel by kernel: the first starts at once and the
+    // launches hide behind the kernels, where graphs of one and two steps
+    // started each about 5 us after the one before (five steps of a 64^3
+    // droplet with readback 215 -> 208 us)
+    cudaGetLastError();  // an earlier call's error is not this launch's
+    for (; left > 0; --left) {
+        s->eng->enqueue_step(s->parity, s->stream);
+        s->parity ^= 1;
+        s->step += 1;
     }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "step launch");
     return PFLBM_OK;
 }
 
 int pflbm_synchronize(pflbm_sim *s) {
     if (!s) return fail(PFLBM_ERR_INVALID_ARG, "null simulation");
-    cudaError_t e = cudaStreamSynchronize(s->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
-    int rc = check_device_error(s);
-    if (rc) return rc;
+    if (const int rc = synchronize(s)) return rc;
     return join_writer(s);
 }
 
@@ -704,7 +730,7 @@ int pflbm_step_profiled(pflbm_sim *s, uint64_t n, double *total_ms, double *kern
     for (auto &x : ev) cudaEventDestroy(x);
     if (e != cudaSuccess) return cuda_fail(e, "pflbm_step_profiled");
     for (int k = 0; k < nk; ++k) kernel_ms[k] = k < 2 ? sums[k] : 0.0;
-    return check_device_error(s);
+    return synchronize(s);
 }
 
 int pflbm_current_step(const pflbm_sim *s, uint64_t *step) {
@@ -778,13 +804,7 @@ int pflbm_set_closure(pflbm_sim *s, const float *blob, float strength) {
     if (rc) return fail(rc, err);
     // steps are captured with the collide kernel of the current mode
     destroy_graphs(s);
-    const int counts[3] = {1, 2, kChunk};
-    for (int par = 0; par < 2; ++par)
-        for (int k = 0; k < 3; ++k) {
-            rc = capture(s, par, counts[k], &s->graphs[par][k]);
-            if (rc) return rc;
-        }
-    return PFLBM_OK;
+    return capture_graphs(s);
 }
 
 
