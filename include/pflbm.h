@@ -253,8 +253,9 @@ int pflbm_load_checkpoint(pflbm_sim *sim, const char *path);
 /* Device bytes held by the simulation. */
 int pflbm_device_bytes(const pflbm_sim *sim, uint64_t *bytes);
 
-/* 1 when the collide kernel is fed by TMA bulk tensor copies (needs
- * 16-byte aligned rows: nx*element size % 16 == 0), 0 for plain loads. */
+/* 1 when the collide kernel is fed by TMA bulk tensor copies, 0 for plain
+ * loads. Rows whose bytes are not a multiple of 16 are padded on the device
+ * for it; where the padded arrays do not fit, the loads are plain. */
 int pflbm_uses_tma(const pflbm_sim *sim, int32_t *flag);
 
 /* Which collide kernel the plain time step runs (the averaging and closure
