@@ -783,7 +783,7 @@ __device__ __forceinline__ void adam_update(float g, float lr, float beta1, floa
 // short (a few us) and strictly serial, so launches and a sum over the blocks
 // by a few threads were most of it. Here every CTA keeps its place: gradient
 // of its blocks into its row of gsum, grid barrier, Adam on the 16 parameters
-// that the CTA owns (moments in registers), grid barrier, the new blob as
+// that the CTA owns, grid barrier, the new blob as
 // fragments. The next iteration's samples do not depend on the parameters and
 // are fetched while the CTA waits at the first barrier. 16 384 samples per iteration: 36 us
 // (two launches) -> 11.7 us, about half of it the block, the rest its FP64 row,
@@ -805,10 +805,6 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_mlp_train(const __grid_consta
     extern __shared__ __align__(16) float tcs[];
     __shared__ double red[kTcThreads];
     __shared__ int s_ok;
-    const int p = blockIdx.x * kSumP + threadIdx.x;
-    const bool owner = threadIdx.x < kSumP && p < kMlpParams;
-    float m = 0.0f, v = 0.0f, w = 0.0f;
-    if (owner) m = a.m[p], v = a.v[p], w = a.blob[p];
     const int rows_used = min(int(gridDim.x), a.blocks);  // the CTAs that have a block
     const bool has = int(blockIdx.x) < a.blocks;
     TcRows rows{};
@@ -833,20 +829,27 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_mlp_train(const __grid_consta
         pflbm::grid_arrive(a.arrived);
         if (has && it + 1 < a.iterations) rows = tc_fetch(a.X, a.Y, a.n, 1, a.seed, a.iter0 + it + 1, a.count, blockIdx.x);
         if (!pflbm::grid_wait(a.arrived, gridDim.x, 2 * it, a.err, &s_ok)) return;
-        if (blockIdx.x < kSumCtas) {
-            const double s = tc_sum_rows(a.gsum, rows_used, blockIdx.x * kSumP, red);
+        // 16 parameters per CTA (more where fewer CTAs than that are resident)
+        for (int c = blockIdx.x; c < kSumCtas; c += gridDim.x) {
+            const int p = c * kSumP + threadIdx.x;
+            const bool owner = threadIdx.x < kSumP && p < kMlpParams;
+            float m = 0.0f, v = 0.0f, w = 0.0f;
+            if (owner) m = a.m[p], v = a.v[p], w = __ldcg(a.blob + p);
+            const double s = tc_sum_rows(a.gsum, rows_used, c * kSumP, red);
             if (owner) {
                 const float g = float(s) * a.inv_count;
                 adam_update(g, a.lr, a.beta1, a.beta2, a.eps, a.c1[it], a.c2[it], m, v, w);
+                a.m[p] = m;
+                a.v[p] = v;
                 __stcg(a.blob + p, w);
             } else if (threadIdx.x < kSumP && p == kMlpParams) {
                 a.loss_log[a.log0 + it] = s * a.inv_count;
             }
+            if (c + int(gridDim.x) < kSumCtas) __syncthreads();  // red is written again
         }
         pflbm::grid_arrive(a.arrived);
         if (!pflbm::grid_wait(a.arrived, gridDim.x, 2 * it + 1, a.err, &s_ok)) return;
     }
-    if (owner) a.m[p] = m, a.v[p] = v;
 }
 
 // ---- the FP32 CUDA-core kernel's sums (PFLBM_MLP_SIMT=1)
@@ -1025,10 +1028,10 @@ void launch_grad_simt(pflbm_closure *c, int blocks, int mode, uint64_t seed, uin
 }
 
 // Iterations it0 .. it0 + k - 1 of a training call in one cooperative launch:
-// one CTA per block as far as they are all resident, and never fewer than
-// own all parameters.
+// one CTA per block and at least one per 16 parameters, as far as they are
+// all resident.
 cudaError_t launch_train(pflbm_closure *c, TrainArgs &a) {
-    const int grid = std::max(kSumCtas, std::min(a.blocks, c->train_ctas));
+    const int grid = std::min(std::max(kSumCtas, a.blocks), c->train_ctas);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kTcThreads);
@@ -1084,7 +1087,7 @@ int pflbm_closure_create(int32_t device, uint64_t max_samples, pflbm_closure **o
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&grad, k_mlp_grad_tc, kTcThreads, kTcSmem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&train, k_mlp_train, kTcThreads, kTcSmem) != cudaSuccess ||
-        grad < 1 || sms * train < kSumCtas)
+        grad < 1 || train < 1)
         return cuda_fail(cudaGetLastError(), "training kernel occupancy");
     c->grad_ctas = sms * grad;
     c->train_ctas = sms * train;
