@@ -15,10 +15,12 @@ namespace pflbm {
 // -------------------------------------------------------------- k_phase
 // phi^{n+1} (computePhase of the next step, src/phaseField.cuh:31-52),
 // outflow rebuild (BoundaryConditions.cuh:107-169) and step counter.
+// Several threads may share a node of a jet's boundary plane: each rebuilds
+// the directions of its mask, and the one that is `first` does the rest.
 template <int QQ, bool JET, class S>
 __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p,
                                            const StepBuffers<S, typename Store<S>::T> &b, int x, int y, int z,
-                                           uint32_t t) {
+                                           uint32_t t, uint32_t mask = ~0u, bool first = true) {
     using T = typename Store<S>::T;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const uint64_t px = p.px;
@@ -66,7 +68,7 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
     }
     T s = T(0);
     s += g0; s += g1; s += g2; s += g3; s += g4; s += g5; s += g6;
-    if (PFLBM_GUARD(X < N, b.err)) b.phi_dst[X] = s;
+    if (first && PFLBM_GUARD(X < N, b.err)) b.phi_dst[X] = s;
 
     if constexpr (JET) {
         if (z == 1) {
@@ -82,9 +84,10 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
             mX.pxx = bp[3 * plane + cX]; mX.pyy = bp[4 * plane + cX]; mX.pzz = bp[5 * plane + cX];
             mX.pxy = bp[6 * plane + cX]; mX.pxz = bp[7 * plane + cX]; mX.pyz = bp[8 * plane + cX];
             const CollideCtx<T> kX = make_ctx<QQ, T>(mX, T(0), T(0), T(0), T(0));
+            int k = 0;  // running index of the rebuilt directions
 #pragma unroll
             for (int q = 1; q < QQ; ++q) {
-                if (kCZ[q] == 1) {
+                if (kCZ[q] == 1 && ((mask >> k++) & 1u)) {
                     const int gx = x - kCX[q], gy = y - kCY[q];
                     if (in_disc<T>(p, gx, gy)) {
                         T bux, buy, buz;
@@ -100,7 +103,7 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
         if (z == nz - 2) {
             // ghost phi of the outlet plane takes this step's value
             // (BoundaryConditions.cuh:127)
-            if (PFLBM_GUARD(idx(x, y, nz - 1) < N, b.err)) b.phi_dst[idx(x, y, nz - 1)] = phiX;
+            if (first && PFLBM_GUARD(idx(x, y, nz - 1) < N, b.err)) b.phi_dst[idx(x, y, nz - 1)] = phiX;
             // outflow rebuild of the populations entering (x,y,nz-2) from
             // the ghost plane: equilibrium of the in-plane source column
             // (x-cx, y-cy), non-equilibrium and force of this node.
@@ -113,9 +116,10 @@ __device__ __forceinline__ void phase_node(const Params<typename Store<S>::T> &p
             mX.pxy = tp[7 * plane + cX]; mX.pxz = tp[8 * plane + cX]; mX.pyz = tp[9 * plane + cX];
             const T fxX = tp[10 * plane + cX], fyX = tp[11 * plane + cX], fzX = tp[12 * plane + cX];
             const CollideCtx<T> kX = make_ctx<QQ, T>(mX, fxX, fyX, fzX, T(0));
+            int k = 0;
 #pragma unroll
             for (int q = 1; q < QQ; ++q) {
-                if (kCZ[q] == -1) {
+                if (kCZ[q] == -1 && ((mask >> k++) & 1u)) {
                     const int bx = wrapi(x - kCX[q], nx), by = wrapi(y - kCY[q], ny);
                     const uint64_t cb = static_cast<uint64_t>(bx) + px * by;
                     const T rb = tp[cb], uxb = tp[plane + cb], uyb = tp[2 * plane + cb], uzb = tp[3 * plane + cb];
@@ -152,8 +156,21 @@ __global__ void __launch_bounds__(256) k_phase(const Params<typename Store<S>::T
 // code does not set the register budget of the vectorised interior path.
 template <int QQ, bool JET, class S>
 __device__ __noinline__ void phase_node_outlined(const Params<float> &p, const StepBuffers<S, float> &b, int x, int y,
-                                                 int z, uint32_t t) {
-    phase_node<QQ, JET, S>(p, b, x, y, z, t);
+                                                 int z, uint32_t t, uint32_t mask, bool first) {
+    phase_node<QQ, JET, S>(p, b, x, y, z, t, mask, first);
+}
+
+// Threads per boundary-plane node. The outflow's relaxation takes an FP64
+// division per rebuilt direction, and a block of 256 nodes with all their
+// directions keeps one SM's FP64 unit (2 lanes per clock) busy for longer than
+// the whole interior of a small grid takes. There a thread per direction
+// shares the node (64x64x128 D3Q19: 6.4 -> 4.6 us); it does where the blocks
+// of a plane, one per direction, fit on the chip's SMs. On larger planes the
+// repeated loads of the node cost more than the wait (101x93x251 D3Q27 15.5 ->
+// 18.5 us with nine threads, 16.1 with two; 128x128x512 40.1 -> 44.4).
+inline int rebuild_groups(int q, uint64_t nx, uint64_t ny, int sms) {
+    const uint64_t blocks = (nx * ny + 255) / 256, directions = q == 19 ? 5 : 9;
+    return blocks * directions <= uint64_t(sms) ? int(directions) : 1;
 }
 
 // The phase sum of the 4 consecutive nodes x4 .. x4+3 of row (y, z), an
@@ -232,7 +249,7 @@ __device__ __forceinline__ void phase_vec4(const Params<float> &p, const StepBuf
 // per thread, in grid slices of their own.
 template <int QQ, bool JET, class S>
 __global__ void __launch_bounds__(256, 4)
-    k_phase_v4(const __grid_constant__ Params<float> p, const __grid_constant__ StepBuffers<S, float> b) {
+    k_phase_v4(const __grid_constant__ Params<float> p, const __grid_constant__ StepBuffers<S, float> b, int G) {
     pdl_release_next();
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const int x4 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
@@ -242,16 +259,21 @@ __global__ void __launch_bounds__(256, 4)
         *b.step_out = *b.step_in + 1ull;
     int z = blockIdx.z;
     if constexpr (JET) {
-        // grid.z = nz + 4: slices 0-3 and 4-7 are the boundary planes 1 and
-        // nz-2, one node per thread (x = x4 + slice), scheduled first because
-        // their rebuilds are the longest; slices 8.. are planes 2 .. nz-3
-        if (blockIdx.z < 8) {
-            const int zb = blockIdx.z < 4 ? 1 : nz - 2;
-            const int x = x4 + (blockIdx.z & 3);
-            if (x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2) phase_node_outlined<QQ, JET, S>(p, b, x, y, zb, t);
+        // grid.z = nz - 4 + 8 G: slices 0 .. 4G-1 and 4G .. 8G-1 are the
+        // boundary planes 1 and nz-2, G threads per node (x = x4 + slice % 4),
+        // scheduled first because their rebuilds are the longest; the others
+        // are planes 2 .. nz-3
+        if (int(blockIdx.z) < 8 * G) {
+            const bool in = int(blockIdx.z) < 4 * G;
+            const int slice = int(blockIdx.z) - (in ? 0 : 4 * G), g = slice >> 2;
+            const int x = x4 + (slice & 3);
+            uint32_t mask = 0u;
+            for (int k = g; k < 9; k += G) mask |= 1u << k;
+            if (x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2)
+                phase_node_outlined<QQ, JET, S>(p, b, x, y, in ? 1 : nz - 2, t, mask, g == 0);
             return;
         }
-        z = blockIdx.z - 6;
+        z = int(blockIdx.z) - 8 * G + 2;
     }
     if (x4 >= nx || y < 1 || y > ny - 2 || z < 1 || z > nz - 2) return;
     phase_vec4<JET, S>(p, b, x4, y, z);
