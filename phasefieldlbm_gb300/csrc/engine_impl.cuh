@@ -396,7 +396,8 @@ class EngineT final : public Engine {
         if (ev) cudaEventRecord(ev[2], s);
         if constexpr (std::is_same<T, float>::value) {
             // (the grid's z extent is limited to 65535)
-            const int groups = JET ? rebuild_groups(QQ, h_.nx, h_.ny, h_.sms) : 1;
+            int groups = JET ? rebuild_groups(QQ, h_.nx, h_.ny, h_.sms) : 1;
+            if (h_.nz - 4 + 8 * groups > 65535) groups = 1;
             const uint32_t gz = JET ? h_.nz - 4 + 8 * groups : h_.nz;
             if (p_.px % 4 == 0 && !no_vec_ && gz <= 65535) {
                 const dim3 blk = phase_block(), g4(((h_.nx + 3) / 4 + blk.x - 1) / blk.x, (h_.ny + blk.y - 1) / blk.y, gz);
