@@ -260,15 +260,17 @@ bool base_field(int32_t id) {
 // Enqueues what brings the cache up to date; its readers follow on the stream.
 int ensure_cache(pflbm_sim *s, bool full = false) {
     if (full) s->wants_full = true;
-    // at step 0 the cache still holds the initial fields
+    // at step 0 the cache still holds the initial fields, or all 18 arrays of
+    // a checkpoint: nothing read there overwrites what the caller may still set
     if (s->cache_step == int64_t(s->step) && (s->cache_full || !full)) return PFLBM_OK;
+    const bool all = s->wants_full || s->step == 0;
     cudaGetLastError();  // an earlier call's error is not this launch's
-    s->eng->enqueue_analysis(s->parity ^ 1, uint32_t(s->step - 1), s->wants_full, s->stream);
+    s->eng->enqueue_analysis(s->parity ^ 1, uint32_t(s->step - 1), all, s->stream);
     s->eng->enqueue_vorticity(s->stream);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "analysis");
     s->cache_step = int64_t(s->step);
-    s->cache_full = s->wants_full;
+    s->cache_full = all;
     return PFLBM_OK;
 }
 
@@ -610,6 +612,7 @@ int pflbm_set_initial_field(pflbm_sim *s, int32_t id, const float *src, size_t b
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy H2D");
     s->distros_dirty = true;
     s->cache_step = 0;
+    s->cache_full = true;
     return PFLBM_OK;
 }
 
@@ -998,6 +1001,7 @@ int pflbm_load_checkpoint(pflbm_sim *s, const char *path) {
     s->parity = 0;
     s->step = h.step;
     s->cache_step = -1;
+    s->cache_full = false;
     s->distros_dirty = false;
     s->initialized = true;
     return PFLBM_OK;
