@@ -148,5 +148,13 @@ def build_dead_grid(jobs: int | None = None) -> Path:
     return build_variant("deadgrid", ["-DPFLBM_TEST_DEAD_GRID"], jobs)
 
 
+def build_fail_launch(jobs: int | None = None) -> Path:
+    """A test build with -DPFLBM_TEST_FAIL_LAUNCH: while PFLBM_FAIL_LAUNCH=1 is
+    set, launches that go through launch_grid (csrc/faults.h) ask for an empty
+    grid, which the runtime refuses with an error code
+    (_build/faillaunch/libpflbm.so)."""
+    return build_variant("faillaunch", ["-DPFLBM_TEST_FAIL_LAUNCH"], jobs)
+
+
 if __name__ == "__main__":
     print(build(verbose=True, force=True))

@@ -211,11 +211,17 @@ int capture(pflbm_sim *s, int parity, int nsteps, cudaGraphExec_t *out) {
     cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
     int p = parity;
-    for (int i = 0; i < nsteps; ++i) {
-        s->eng->enqueue_step(p, s->stream);
+    cudaGetLastError();  // an earlier call's error is not this launch's
+    cudaError_t le = cudaSuccess;
+    for (int i = 0; i < nsteps && le == cudaSuccess; ++i) {
+        le = s->eng->enqueue_step(p, s->stream);
         p ^= 1;
     }
     e = cudaStreamEndCapture(s->stream, &graph);
+    if (le != cudaSuccess) {
+        if (e == cudaSuccess) cudaGraphDestroy(graph);
+        return cuda_fail(le, "step capture");
+    }
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
     e = cudaGraphInstantiate(out, graph, 0);
     cudaGraphDestroy(graph);
@@ -635,12 +641,11 @@ int pflbm_step_async(pflbm_sim *s, uint64_t n) {
     // droplet with readback 215 -> 208 us)
     cudaGetLastError();  // an earlier call's error is not this launch's
     for (; left > 0; --left) {
-        s->eng->enqueue_step(s->parity, s->stream);
+        const cudaError_t e = s->eng->enqueue_step(s->parity, s->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "step launch");
         s->parity ^= 1;
         s->step += 1;
     }
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(e, "step launch");
     return PFLBM_OK;
 }
 
@@ -711,14 +716,18 @@ int pflbm_step_profiled(pflbm_sim *s, uint64_t n, double *total_ms, double *kern
                 if (y) cudaEventDestroy(y);
             return cuda_fail(cudaGetLastError(), "cudaEventCreate");
         }
+    cudaGetLastError();  // an earlier call's error is not this launch's
     cudaEventRecord(ev[0], s->stream);
+    cudaError_t le = cudaSuccess;
     for (uint64_t i = 0; i < n; ++i) {
-        s->eng->enqueue_step(s->parity, s->stream, &ev[1 + i * kEv]);
+        le = s->eng->enqueue_step(s->parity, s->stream, &ev[1 + i * kEv]);
+        if (le != cudaSuccess) break;
         s->parity ^= 1;
         s->step += 1;
     }
     cudaEventRecord(ev.back(), s->stream);
     cudaError_t e = cudaEventSynchronize(ev.back());
+    if (e == cudaSuccess) e = le;
     double sums[2] = {0.0, 0.0};
     float ms = 0.0f;
     if (e == cudaSuccess) {

@@ -41,7 +41,9 @@ class Engine {
     virtual void free_all() = 0;
     // Enqueues one time step reading ping-pong buffer `parity`. With
     // events (2 per kernel) the kernels are bracketed by event records.
-    virtual void enqueue_step(int parity, cudaStream_t s, cudaEvent_t *events = nullptr) = 0;
+    // Returns the error of a launch that failed; the step then has not run
+    // (the caller clears cudaGetLastError() before the first step).
+    virtual cudaError_t enqueue_step(int parity, cudaStream_t s, cudaEvent_t *events = nullptr) = 0;
     // Initial macroscopic fields into the cache, then f/phi from them.
     virtual void enqueue_init_fields(cudaStream_t s) = 0;
     virtual void enqueue_init_distros(cudaStream_t s) = 0;

@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "engine.h"
+#include "faults.h"
 #include "kernels.cuh"
 #include "kernels_pair.cuh"
 #include "kernels_tma.cuh"
@@ -319,7 +320,7 @@ class EngineT final : public Engine {
     dim3 collide_grid(const Params<T> &p) const {
         const int nzi = int(h_.nz) - 2;
         const int chunks = (nzi + p.zchunk - 1) / p.zchunk;
-        return dim3((h_.nx + TX - 1) / TX, (h_.ny + TY - 1) / TY, chunks);
+        return launch_grid(dim3((h_.nx + TX - 1) / TX, (h_.ny + TY - 1) / TY, chunks));
     }
     dim3 node_block() const { return dim3(32, 8, 1); }
     // Block of the float4 phase step: 32, 16 or 8 segments of 4 nodes along x,
@@ -356,7 +357,7 @@ class EngineT final : public Engine {
         cudaLaunchKernelEx(&cfg, kernel, args...);
     }
 
-    void enqueue_step(int parity, cudaStream_t s, cudaEvent_t *ev) override {
+    cudaError_t enqueue_step(int parity, cudaStream_t s, cudaEvent_t *ev) override {
         const StepBuffers<S, T> b = buffers(parity);
         if (ev) cudaEventRecord(ev[0], s);
         if (closure_) {
@@ -392,6 +393,8 @@ class EngineT final : public Engine {
         } else {
             k_collide<QQ, JET, S, MODE_STEP><<<collide_grid(), dim3(TX, TY, 1), 0, s>>>(p_, b);
         }
+        // no phase step behind a collide that did not start
+        if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
         if (ev) cudaEventRecord(ev[1], s);
         if (ev) cudaEventRecord(ev[2], s);
         if constexpr (std::is_same<T, float>::value) {
@@ -409,6 +412,7 @@ class EngineT final : public Engine {
             k_phase<QQ, JET, S><<<node_grid(), node_block(), 0, s>>>(p_, b);
         }
         if (ev) cudaEventRecord(ev[3], s);
+        return cudaGetLastError();
     }
 
     InitGeom geom() const {
