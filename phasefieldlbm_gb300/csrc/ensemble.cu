@@ -504,27 +504,35 @@ class Ensemble {
 
     // Analysis of one box after the last completed step into the macro cache:
     // all 18 arrays (`full`) or those of MODE_ANALYSIS_BASE. The cache holds
-    // one box at a time; a field of the box that it holds is read from it.
+    // one box at a time; a field of the box that it holds is read from it. It
+    // holds nothing from the first launch on until all have been accepted.
     int cache_box = -1;
     uint64_t cache_step = 0;
     bool cache_full = false;
-    void enqueue_analysis_box(int k, bool full) {
-        if (cache_box == k && cache_step == step && (cache_full || !full)) return;
+    cudaError_t enqueue_analysis_box(int k, bool full) {
+        if (cache_box == k && cache_step == step && (cache_full || !full)) return cudaSuccess;
+        cache_box = -1;
+        cudaGetLastError();  // an earlier call's error is not this launch's
+        if (step == 0)
+            enqueue_init_box(k);  // the cache then holds the initial fields
+        else
+            launch_analysis_box(k, full);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
         cache_box = k;
         cache_step = step;
         cache_full = full || step == 0;
+        return cudaSuccess;
+    }
+    void launch_analysis_box(int k, bool full) {
         const Params<float> &p = boxes[k].p;
-        if (step == 0) {
-            enqueue_init_box(k);  // the cache then holds the initial fields
-            return;
-        }
         StepBuffers<float, float> b = host_box_buffers(k, parity ^ 1);
         b.f_dst = nullptr;
         b.phi_dst = nullptr;
         b.step_in = nullptr;
         b.t_fixed = uint32_t(step - 1);
         const int chunks = (int(p.nz) - 2 + p.zchunk - 1) / p.zchunk;
-        const dim3 cg((p.nx + TX - 1) / TX, (p.ny + TY - 1) / TY, chunks);
+        const dim3 cg = launch_grid(dim3((p.nx + TX - 1) / TX, (p.ny + TY - 1) / TY, chunks));
         const dim3 blk3(TX, TY);
         if (full && q == 19)
             k_collide<19, false, float, MODE_ANALYSIS><<<cg, blk3, 0, stream>>>(p, b);
@@ -700,9 +708,9 @@ int pflbm_ensemble_get_field(pflbm_ensemble *e, int32_t box, int32_t id, void *h
     cudaSetDevice(e->device);
     const bool base = id == PFLBM_FIELD_RHO || id == PFLBM_FIELD_UX || id == PFLBM_FIELD_UY || id == PFLBM_FIELD_UZ ||
                       id == PFLBM_FIELD_PHI || id == PFLBM_FIELD_IND;
-    e->enqueue_analysis_box(box, !base);
-    const cudaError_t ce =
-        cudaMemcpyAsync(host, e->macro + size_t(id) * N, N * sizeof(float), cudaMemcpyDeviceToHost, e->stream);
+    cudaError_t ce = e->enqueue_analysis_box(box, !base);
+    if (ce != cudaSuccess) return ecuda(ce, "ensemble analysis");
+    ce = cudaMemcpyAsync(host, e->macro + size_t(id) * N, N * sizeof(float), cudaMemcpyDeviceToHost, e->stream);
     if (ce != cudaSuccess) return ecuda(ce, "ensemble readback");
     const cudaError_t se = cudaStreamSynchronize(e->stream);
     if (se != cudaSuccess) return ecuda(se, "ensemble readback");
@@ -713,13 +721,14 @@ int pflbm_ensemble_reduce(pflbm_ensemble *e, int32_t box, pflbm_diag *d) {
     if (!e || !d) return efail(PFLBM_ERR_INVALID_ARG, "null argument");
     if (box < 0 || box >= int32_t(e->boxes.size())) return efail(PFLBM_ERR_INVALID_ARG, "box index out of range");
     cudaSetDevice(e->device);
-    e->enqueue_analysis_box(box, false);
+    cudaError_t ce = e->enqueue_analysis_box(box, false);
+    if (ce != cudaSuccess) return ecuda(ce, "ensemble analysis");
     pflbm::k_reduce_partial<float><<<Ensemble::kRedBlocks, pflbm::RED_THREADS, 0, e->stream>>>(e->boxes[box].p, e->macro,
                                                                                                e->partial);
     pflbm::k_reduce_final<<<1, pflbm::RED_FINAL_THREADS, 0, e->stream>>>(e->partial, Ensemble::kRedBlocks, e->dev_diag);
     double r[12];
     cudaMemcpyAsync(r, e->dev_diag, sizeof r, cudaMemcpyDeviceToHost, e->stream);
-    const cudaError_t ce = cudaStreamSynchronize(e->stream);
+    ce = cudaStreamSynchronize(e->stream);
     if (ce != cudaSuccess) return ecuda(ce, "ensemble reduce");
     std::memset(d, 0, sizeof(*d));
     d->step = e->step;

@@ -53,3 +53,20 @@ def test_steps_that_were_not_launched_do_not_count(pflbm, failing, vs, storage, 
         s.step(33 - done)
         for f in fields:
             assert np.array_equal(s.get_field(f, dtype=np.float64), want[f]), f
+
+
+def test_ensemble_readback_that_was_not_launched_is_not_served(pflbm, failing):
+    cfgs = [droplet_cfg(pflbm, 19, n=n, radius=6) for n in (32, 36)]
+    with pflbm.Ensemble(cfgs) as e:
+        e.step(7)
+        want = {(k, f): e.get_field(k, f) for k in (0, 1) for f in ("phi", "pxy")}
+    with pflbm.Ensemble(cfgs) as e:
+        e.get_field(1, "phi")
+        e.step(7)
+        failing(True)
+        for k, f in want:
+            _refused(pflbm, lambda: e.get_field(k, f))
+        _refused(pflbm, lambda: e.reduce(1))
+        failing(False)
+        for (k, f), a in want.items():
+            assert np.array_equal(e.get_field(k, f), a), (k, f)
