@@ -353,7 +353,10 @@ int pflbm_closure_set_blob(pflbm_closure *c, const float *host_blob);
  * count samples, FP64 accumulation of FP32 per-block sums. */
 int pflbm_closure_gradient(pflbm_closure *c, uint64_t count, double *host_grad, double *loss_sum);
 /* Adam (beta 0.9/0.999, eps 1e-8) on minibatches drawn by a counter hash;
- * loss_history (may be NULL) receives the mean minibatch loss per iteration. */
+ * loss_history (may be NULL) receives the mean minibatch loss per iteration.
+ * After PFLBM_ERR_DEVICE (a wait inside the kernel gave up) the parameters are
+ * those of no known iteration: train, gradient and loss return PFLBM_ERR_STATE
+ * until set_blob or init_params. */
 int pflbm_closure_train(pflbm_closure *c, int32_t iterations, int32_t batch, float lr, uint32_t seed,
                         double *loss_history);
 int pflbm_closure_loss(pflbm_closure *c, double *mean_loss);

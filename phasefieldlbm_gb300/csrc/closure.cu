@@ -45,6 +45,7 @@
 
 #include "../../include/pflbm.h"
 #include "engine.h"
+#include "faults.h"
 #include "gridbar.cuh"
 #include "kernels.cuh"
 #include "packed.cuh"
@@ -805,6 +806,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_mlp_train(const __grid_consta
     extern __shared__ __align__(16) float tcs[];
     __shared__ double red[kTcThreads];
     __shared__ int s_ok;
+    // behind a launch whose barrier ran out nothing moves any more
+    if (__syncthreads_or(__ldcg(a.err) != 0u)) return;
     const int rows_used = min(int(gridDim.x), a.blocks);  // the CTAs that have a block
     const bool has = int(blockIdx.x) < a.blocks;
     TcRows rows{};
@@ -1033,7 +1036,7 @@ void launch_grad_simt(pflbm_closure *c, int blocks, int mode, uint64_t seed, uin
 cudaError_t launch_train(pflbm_closure *c, TrainArgs &a) {
     const int grid = std::min(std::max(kSumCtas, a.blocks), c->train_ctas);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = pflbm::launch_grid(dim3(grid));
     cfg.blockDim = dim3(kTcThreads);
     cfg.dynamicSmemBytes = kTcSmem;
     cfg.stream = c->stream;
@@ -1321,28 +1324,34 @@ int pflbm_closure_train(pflbm_closure *c, int32_t iterations, int32_t batch, flo
         a.inv_count = 1.0f / float(batch), a.lr = lr, a.beta1 = beta1, a.beta2 = beta2, a.eps = eps;
         a.gsum = c->gsum, a.loss_log = c->loss_log, a.arrived = c->sync, a.err = c->sync + 1;
         cudaMemsetAsync(c->sync, 0, 2 * sizeof(unsigned int), c->stream);
-        for (int it = 0; it < iterations; it += kTrainChunk) {
-            a.iterations = std::min(kTrainChunk, iterations - it);
-            a.iter0 = c->adam_t + 1;
-            a.log0 = it;
+        int launched = 0;  // iterations; they count when they have run
+        cudaError_t le = cudaSuccess;
+        while (launched < iterations) {
+            a.iterations = std::min(kTrainChunk, iterations - launched);
+            a.iter0 = c->adam_t + launched + 1;
+            a.log0 = launched;
             for (int k = 0; k < a.iterations; ++k) {
                 a.c1[k] = correction(beta1, a.iter0 + k);
                 a.c2[k] = correction(beta2, a.iter0 + k);
             }
-            c->adam_t += a.iterations;
-            if (it > 0) cudaMemsetAsync(c->sync, 0, sizeof(unsigned int), c->stream);
-            const cudaError_t le = launch_train(c, a);
-            if (le != cudaSuccess) return cuda_fail(le, "training launch");
+            if (launched > 0) cudaMemsetAsync(c->sync, 0, sizeof(unsigned int), c->stream);
+            le = launch_train(c, a);
+            if (le != cudaSuccess) break;  // what was launched before still counts
+            launched += a.iterations;
         }
+        cudaError_t e = cudaStreamSynchronize(c->stream);
+        unsigned int w = 0;
+        if (e == cudaSuccess) e = cudaMemcpy(&w, c->sync + 1, sizeof w, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess || w != 0) c->have_params = false;  // of no known iteration
+        if (e != cudaSuccess) return cuda_fail(e, "closure training");
+        if (w)
+            return fail(PFLBM_ERR_DEVICE,
+                        "the training kernel gave up waiting at its grid barrier; set or initialise the parameters again");
+        c->adam_t += launched;
+        if (le != cudaSuccess) return cuda_fail(le, "training launch");
     }
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "closure training");
-    if (!simt) {
-        unsigned int w = 0;
-        e = cudaMemcpy(&w, c->sync + 1, sizeof w, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return cuda_fail(e, "closure training");
-        if (w) return fail(PFLBM_ERR_DEVICE, "the training kernel gave up waiting at its grid barrier");
-    }
     if (loss_history) {
         e = cudaMemcpy(loss_history, c->loss_log, sizeof(double) * iterations, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(e, "loss history");

@@ -70,3 +70,21 @@ def test_ensemble_readback_that_was_not_launched_is_not_served(pflbm, failing):
         failing(False)
         for (k, f), a in want.items():
             assert np.array_equal(e.get_field(k, f), a), (k, f)
+
+
+def test_training_that_was_not_launched_does_not_count(pflbm, failing):
+    x = _features(3000, 51)
+    y = _targets(x, 52)
+    blobs = []
+    for interrupted in (False, True):
+        with pflbm.Closure(3000) as c:
+            c.set_samples(x, y)
+            c.init_params(seed=3)
+            c.train(40, batch=700, lr=2e-3, seed=5)
+            if interrupted:
+                failing(True)
+                _refused(pflbm, lambda: c.train(300, batch=700, lr=2e-3, seed=5))
+                failing(False)
+            c.train(40, batch=700, lr=2e-3, seed=5)
+            blobs.append(c.blob.copy())
+    assert np.array_equal(*blobs)
