@@ -133,11 +133,17 @@ def build_checked(jobs: int | None = None) -> Path:
 
 
 def build_dead_wait(jobs: int | None = None) -> Path:
-    """A test build with -DPFLBM_TEST_DEAD_WAIT: the collide pipelines' first
-    wait of every plane polls an mbarrier that nothing arrives on, with a
+    """A test build with -DPFLBM_TEST_DEAD_WAIT: the collide pipelines' wait
+    for a plane polls an mbarrier that nothing arrives on, with a
     short limit, so that the bounded wait runs out and the kernel reports
     through the device error word and returns (_build/deadwait/libpflbm.so)."""
     return build_variant("deadwait", ["-DPFLBM_TEST_DEAD_WAIT"], jobs)
+
+
+def build_dead_warmup(jobs: int | None = None) -> Path:
+    """The same with -DPFLBM_TEST_DEAD_WARMUP for the wait for a tile's first
+    phi planes (_build/deadwarmup/libpflbm.so)."""
+    return build_variant("deadwarmup", ["-DPFLBM_TEST_DEAD_WARMUP"], jobs)
 
 
 def build_dead_grid(jobs: int | None = None) -> Path:

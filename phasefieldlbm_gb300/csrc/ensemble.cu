@@ -678,7 +678,7 @@ int pflbm_ensemble_step(pflbm_ensemble *e, uint64_t n) {
     if (ce != cudaSuccess) return ecuda(ce, "ensemble step");
     unsigned int w = 0;
     cudaMemcpy(&w, e->bp.err, sizeof w, cudaMemcpyDeviceToHost);
-    if (w) return efail(PFLBM_ERR_DEVICE, "a kernel reported an error");
+    if (w) return efail(PFLBM_ERR_DEVICE, "a kernel reported an error (error word " + std::to_string(w) + ")");
     return PFLBM_OK;
 }
 

@@ -558,12 +558,12 @@ __device__ __forceinline__ bool collide_tile_pair(const Params<float> &p, const 
             if (ly >= 1 && ly <= TY) *reinterpret_cast<float2 *>(&ind_at(zp, ly - 1, lx)) = indv.v;
         }
     };
-    if (!plane_wait<L>(smem, warm_bar<L>(smem), 0)) *s_abort = 1;
+    if (!warm_wait<L>(smem, 0)) *s_abort = 1;
     compute_n(zb - 1);
     __syncthreads();
     if (*s_abort) {
         if (tid == 0) {
-            atomicOr(b.err, 1u);
+            atomicOr(b.err, 8u);
             mbar_wait_bounded(warm_bar<L>(smem), 0, kWaitLimit);
             for (int k = 0; k < NS - 2 && zb + k < ze; ++k)
                 mbar_wait_bounded(&bar[(seq + k) % NS], ((seq + k) / NS) & 1, kWaitLimit);

@@ -213,7 +213,7 @@ __device__ __forceinline__ void tma_pipeline_init(unsigned char *smem) {
         for (int k = 0; k < L::kStages; ++k) mbar_init(&bar[k], 1);
         mbar_init(warm_bar<L>(smem), 1);
         *reinterpret_cast<volatile int *>(smem + L::off_bar + 8 * L::kStages) = 0;
-#ifdef PFLBM_TEST_DEAD_WAIT
+#if defined(PFLBM_TEST_DEAD_WAIT) || defined(PFLBM_TEST_DEAD_WARMUP)
         mbar_init(reinterpret_cast<uint64_t *>(smem + L::off_bar + 64), 1);
 #endif
         fence_mbar_init();
@@ -222,19 +222,32 @@ __device__ __forceinline__ void tma_pipeline_init(unsigned char *smem) {
 }
 
 // The per-plane wait of the collide pipelines: phase `parity` of the stage's
-// barrier, bounded. A test build (-DPFLBM_TEST_DEAD_WAIT, never the shipped
-// library) polls instead a barrier that nothing arrives on, with a short
-// limit, so that the wait always runs out and the failure path (error word,
-// drain of the CTA's own copies at the full limit, return) is exercised.
+// barrier, bounded. Two test builds, never the shipped library, poll instead
+// a barrier that nothing arrives on, with a short limit, so that the wait
+// always runs out and the failure path (error word, drain of the CTA's own
+// copies at the full limit, return) is exercised: -DPFLBM_TEST_DEAD_WAIT this
+// one, -DPFLBM_TEST_DEAD_WARMUP the tile's first wait (warm_wait).
+template <class L>
+__device__ __forceinline__ bool dead_wait(unsigned char *smem) {
+    return mbar_wait_bounded(reinterpret_cast<uint64_t *>(smem + L::off_bar + 64), 0, 1u << 12);
+}
 template <class L>
 __device__ __forceinline__ bool plane_wait(unsigned char *smem, uint64_t *bar, uint32_t parity) {
 #ifdef PFLBM_TEST_DEAD_WAIT
-    (void)bar;
-    (void)parity;
-    return mbar_wait_bounded(reinterpret_cast<uint64_t *>(smem + L::off_bar + 64), 0, 1u << 12);
+    return dead_wait<L>(smem);
 #else
-    (void)smem;
     return mbar_wait_bounded(bar, parity, kWaitLimit);
+#endif
+}
+
+// The wait for a tile's first phi planes. Where it gives up, the error word
+// takes 8, where a plane's wait does, 1.
+template <class L>
+__device__ __forceinline__ bool warm_wait(unsigned char *smem, uint32_t parity) {
+#ifdef PFLBM_TEST_DEAD_WARMUP
+    return dead_wait<L>(smem);
+#else
+    return mbar_wait_bounded(warm_bar<L>(smem), parity, kWaitLimit);
 #endif
 }
 
@@ -367,12 +380,12 @@ __device__ __forceinline__ bool collide_tile_tma(const Params<typename Store<S>:
             }
         }
     };
-    if (!plane_wait<L>(smem, warm_bar<L>(smem), tiles & 1)) *s_abort = 1;
+    if (!warm_wait<L>(smem, tiles & 1)) *s_abort = 1;
     compute_n(zb - 1);
     __syncthreads();
     if (*s_abort) {
         if (tid == 0) {
-            atomicOr(b.err, 1u);
+            atomicOr(b.err, 8u);
             mbar_wait_bounded(warm_bar<L>(smem), tiles & 1, kWaitLimit);
             for (int k = 0; k < NS - 2 && zb + k < ze; ++k)
                 mbar_wait_bounded(&bar[(seq + k) % NS], ((seq + k) / NS) & 1, kWaitLimit);
