@@ -108,19 +108,29 @@ class EngineT final : public Engine {
     // Rows that do not start on 16-byte boundaries are padded, so that every
     // grid runs the TMA-fed collide and the float4 phase step (D3Q27 FP32
     // 101x93x251: collide 205 -> 147 us, phase 55 -> 20 us against the
-    // plain-load kernels).
-    // Where the padded arrays do not fit, the grid keeps its own rows and the
-    // plain-load kernels.
+    // plain-load kernels). FP32 rows are padded to whole 32-byte sectors where
+    // that makes them at most an eighth longer (97x93x251 D3Q27 150 us a step
+    // against 155 with rows of 100, 193x129x300 D3Q19 287 against 309, but 33
+    // wide 50.6 against 49.2); the others to 16 bytes, which takes less memory
+    // at the same speed (16-bit 97, 129, 193 and 257 wide, 33 wide: within 1%).
+    // Where the padded arrays do not fit and leave kPadReserve of the device
+    // free, the grid keeps its own rows and the plain-load kernels: what the
+    // program allocates next finds room where it would without padding.
+    static constexpr uint64_t kPadReserve = uint64_t(256) << 20;
+    uint32_t padded_row() const {
+        auto up = [&](uint32_t unit) { return (h_.nx + unit - 1) / unit * unit; };
+        const uint32_t sectors = up(32 / sizeof(S));
+        return sizeof(S) == 4 && 8 * uint64_t(sectors - h_.nx) <= h_.nx ? sectors : up(16 / sizeof(S));
+    }
     int allocate(std::string &err) override {
-        const uint32_t unit = 32 / sizeof(S);  // 32-byte sectors
         const bool aligned = (uint64_t(h_.nx) * sizeof(S)) % 16 == 0 && (uint64_t(h_.nx) * sizeof(T)) % 16 == 0;
         const char *no_tma = std::getenv("PFLBM_NO_TMA");
-        const uint32_t padded = (h_.nx + unit - 1) / unit * unit;
+        const uint32_t padded = padded_row();
         int rc = PFLBM_ERR_OUT_OF_MEMORY;
         if (!aligned && !(no_tma && no_tma[0] == '1') &&
             uint64_t(padded) * h_.ny * h_.nz < (uint64_t(1) << 32))  // 32-bit node indices
-            rc = allocate_rows(padded, err);
-        if (rc == PFLBM_ERR_OUT_OF_MEMORY) rc = allocate_rows(h_.nx, err);
+            rc = allocate_rows(padded, kPadReserve, err);
+        if (rc == PFLBM_ERR_OUT_OF_MEMORY) rc = allocate_rows(h_.nx, 0, err);
         if (rc) return rc;
         if (cudaDeviceSynchronize() != cudaSuccess) {
             err = cudaGetErrorString(cudaGetLastError());
@@ -131,7 +141,8 @@ class EngineT final : public Engine {
         return PFLBM_OK;
     }
 
-    int allocate_rows(uint32_t px, std::string &err) {
+    // The arrays with rows of px, if they leave `reserve` bytes of the device.
+    int allocate_rows(uint32_t px, uint64_t reserve, std::string &err) {
         const uint64_t Nd = h_.N, plane = uint64_t(px) * h_.ny, N = plane * h_.nz;
         struct Req {
             void **ptr;
@@ -158,11 +169,16 @@ class EngineT final : public Engine {
         for (auto &r : reqs) planned += r.bytes;
         if (const char *lim = std::getenv("PFLBM_ALLOC_LIMIT_BYTES")) {
             const unsigned long long cap = std::strtoull(lim, nullptr, 10);
-            if (cap > 0 && planned > cap) {
+            if (cap > 0 && planned + reserve > cap) {
                 err = "device allocation of " + std::to_string(planned) + " bytes exceeds PFLBM_ALLOC_LIMIT_BYTES=" +
                       std::to_string(cap);
                 return PFLBM_ERR_OUT_OF_MEMORY;
             }
+        }
+        size_t room = 0, total = 0;
+        if (reserve > 0 && cudaMemGetInfo(&room, &total) == cudaSuccess && planned + reserve > room) {
+            err = "no room for padded rows";
+            return PFLBM_ERR_OUT_OF_MEMORY;
         }
         for (auto &r : reqs) {
             if (r.bytes == 0) continue;
