@@ -95,9 +95,10 @@ __device__ __forceinline__ float sigmoidf_(float a) { return __frcp_rn(1.0f + ex
 // Box filter and restriction in FP64, bound by the FP64 unit. A thread owns a
 // coarse column (i, j) of a z chunk, sums every fine plane of its boxes once
 // and carries plane 2k+1 on to the next coarse plane; the floats are widened on
-// the integer units: 251 FP64 instructions per coarse node instead of 455 with
-// the conversions, 64x64x256 coarse nodes 910 -> 560 us (753 with the
-// conversions in FP64).
+// the integer units: 251 FP64 instructions per coarse node by count (275
+// executed, the chunks' first planes included) instead of 455 with the
+// conversions, 64x64x256 coarse nodes 910 -> 560 us (753 with the conversions
+// in FP64).
 constexpr int kFilterX = 32, kFilterY = 4, kFilterPlanes = 8;
 __global__ void __launch_bounds__(kFilterX *kFilterY) k_filter_restrict(const float *__restrict__ macro, uint64_t Nf,
                                                                         int nxf, int nyf, int nzf, int nxc, int nyc,
@@ -386,7 +387,8 @@ __global__ void __launch_bounds__(kSB) k_mlp_grad(const float *__restrict__ blob
 // conflict-free loads instead of 4- and 8-way conflicts and a conversion per
 // use), a sigmoid is evaluated once per unit instead of two or three times,
 // and two warps share what one warp did: 2^20 samples 398 -> 226 us at 16
-// warps per SM (IPC 1.6, 3640 warp instructions per 32 samples), 202 us at 24.
+// warps per SM, 202 us at 24 (3790 warp instructions per 32 samples, 2.1 of 4
+// issued per clock).
 constexpr int kTcThreads = 2 * kSB;
 constexpr int kTcPairs = kSB / 32;
 constexpr int kTcX = 12;         // row stride of the Xn tile (words)

@@ -15,8 +15,8 @@ struct GridBar {
     unsigned int pad;
 };
 
-// Bounded polls of the grid barrier (with a short sleep each: well above any
-// sweep's duration, below a second).
+// Bounded polls of the grid barrier, each a sleep of 64 ns and a load from L2:
+// a few seconds in all, far above the difference between the CTAs of any sweep.
 constexpr uint32_t kGridWaitLimit = 1u << 22;
 
 __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int *p) {

@@ -2,8 +2,8 @@
 //
 // The same algebra as lattice.cuh and stencil.cuh, arranged for the fewest
 // FP64 instructions: the unit has 2 lanes per clock and SM, and an FP64 step
-// keeps it busy 82% of the time while memory and every other pipe idle, so
-// its time is the count of FP64 instructions per node. What is shared:
+// keeps it busy 81% of the time with DRAM at 7% and issue at 8%, so its time
+// is the count of FP64 instructions per node. What is shared:
 //   - the differences of opposite face diagonals serve two gradient axes
 //     (sum and difference), the divergence of the normals takes one weighted
 //     sum instead of three, and the factor 3 sits in the weights;
@@ -13,9 +13,11 @@
 //   - collision: the even part of every direction is w (K + 4.5 c.T.c) with
 //     one tensor T = rho u u + sym(u F) + (1 - omega) Pi, the odd part of
 //     D3Q19 is 3 w c.(rho u + F/2).
-// Every operation is rounded by itself (op_*), so the plain-load and TMA-fed
-// kernels agree bit for bit. D3Q19 jet 96x96x256: 1835 (375 FP64 instructions
-// per node) -> 1340 us per collide; fields within 4e-14 of the direct forms.
+// Every operation but those of the third-order odd part of D3Q27 (make_ctx,
+// cdot, hermite3) is rounded by itself (op_*); the plain-load and TMA-fed
+// kernels agree bit for bit. D3Q19 jet 96x96x256: 375 -> 284 FP64 instructions
+// per interior node (the halo's normals included), 1835 -> 1340 us per collide;
+// fields within 4e-14 of the direct forms.
 #pragma once
 #include "lattice.cuh"
 #include "stencil.cuh"

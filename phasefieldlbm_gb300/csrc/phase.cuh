@@ -245,8 +245,8 @@ __device__ __forceinline__ void phase_vec4(const Params<float> &p, const StepBuf
 // FP32 phase step with 128-bit accesses: one thread owns 4 consecutive x
 // nodes (px % 4 == 0), reads the phi/J rows of its y and z neighbours as
 // float4 and the two x-end neighbours (periodically wrapped) as scalars.
-// The jet's boundary planes z = 1 and nz-2 go through phase_node, one node
-// per thread, in grid slices of their own.
+// The jet's boundary planes z = 1 and nz-2 go through phase_node, G threads
+// per node (rebuild_groups), in grid slices of their own.
 template <int QQ, bool JET, class S>
 __global__ void __launch_bounds__(256, 4)
     k_phase_v4(const __grid_constant__ Params<float> p, const __grid_constant__ StepBuffers<S, float> b, int G) {

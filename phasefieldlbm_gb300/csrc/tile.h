@@ -32,12 +32,16 @@ static_assert(kTileX % 32 == 0 && kTileX * kTileY <= 1024, "collide tile");
 // (which has the SM for itself), and hides less (two planes more). Of the
 // chunks within 6% of the least, the one nearest to 8 planes is taken: what
 // the model calls equal is faster with shorter chunks, whose CTAs read the
-// planes more nearly in order. Against the fastest of a sweep of chunks the
-// choice is 1% slower on average over 22 grids from 32x32x64 to 256x256x1024
-// (every storage type, plain and closure kernels; 4% at most). Eight CTAs per
-// SM at least four planes long, the rule before: FP16 256x256x1024 1859 ->
-// 1494 us, FP32 64x64x128 30.6 -> 22.6, 96^3 46.5 -> 33.1, 128^3 87.1 -> 71.0,
-// of which a fifth to a third is the shorter warm-up.
+// planes more nearly in order. (Not always: the D3Q27 FP32 128x128x512 jet gets
+// 20 planes instead of 27, 364 instead of 358 us.) Against the fastest of a
+// sweep of chunks the choice is 1% slower on average over the 22 grids it was
+// fitted on, 32x32x64 to 256x256x1024 (every storage type, plain and closure
+// kernels; 4% at most), and over 36 random ones that it was not fitted on, up
+// to 16 M nodes, 1.6% in FP32 (10% at most) and 4.8% in 16 bits (23% at most:
+// D3Q19 BF16 97x165x33, 33 instead of 27 us). Eight CTAs per SM at least four
+// planes long, the rule before: FP16 256x256x1024 1859 -> 1494 us, FP32
+// 64x64x128 30.6 -> 22.6, 96^3 46.5 -> 33.1, 128^3 87.1 -> 71.0, of which a
+// fifth to a third is the shorter warm-up.
 inline int pick_zchunk(int tiles, int nzi, int sms, int per_sm) {
     auto planes = [&](int chunks) { return (nzi + chunks - 1) / chunks; };
     auto time = [&](int zc) {
